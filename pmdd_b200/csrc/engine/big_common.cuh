@@ -27,6 +27,13 @@ __device__ __forceinline__ void fill_item(const ExpandJob &J, int64_t k, int64_t
     b->n = J.arc_cand_off[b->a1 - J.arc_base] - b->c0;
 }
 
+// Scratch of the destination at scratch offset soff beside its candidates: 2 * n points'
+// bytes, laid out by whichever path filters it.
+template <int D, typename T>
+__device__ __forceinline__ unsigned char *big_slab(const ExpandJob &J, int64_t soff) {
+    return static_cast<unsigned char *>(J.big_slab) + soff * static_cast<int64_t>(2 * D * sizeof(T));
+}
+
 // Destinations of three objectives whose runs all come from sorted frontiers, at most
 // J.lex_max_arcs of them: the lexicographic path (big_lex.cu) filters these.
 __device__ __forceinline__ bool lex_eligible(const ExpandJob &J, const BigItem &B) {

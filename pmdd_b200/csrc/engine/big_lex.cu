@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kRankThreads) big_lex_rank_kernel(const Expand
 
 // Merge round `round` of the lexicographic destinations with more than kBigDirectArcs
 // runs: at round r the destination consists of sorted groups of 2^r consecutive runs
-// (in big_pts for even r, big_pts2 for odd r); each candidate moves to its place in the
+// (in big_pts for even r, the slab for odd r); each candidate moves to its place in the
 // union with its sibling group (a binary search there; equal points: the left group
 // first), in the other buffer.  Thread per candidate of the scratch pass.
 template <typename T>
@@ -133,8 +133,10 @@ __global__ void __launch_bounds__(kRankThreads) big_lex_merge_kernel(const Expan
         const ExpandJob &J = jobs[c.job];
         const int K = c.B.a1 - c.B.a0;
         if (!J.lex_big || round >= lex_merge_rounds(K) || !lex_eligible(J, c.B)) continue;
-        const T *src = static_cast<const T *>(round & 1 ? J.big_pts2 : J.big_pts) + c.B.soff * 3;
-        T *dst = static_cast<T *>(round & 1 ? J.big_pts : J.big_pts2) + c.B.soff * 3;
+        T *even = static_cast<T *>(J.big_pts) + c.B.soff * 3;
+        T *odd = reinterpret_cast<T *>(big_slab<3, T>(J, c.B.soff));
+        const T *src = round & 1 ? odd : even;
+        T *dst = round & 1 ? even : odd;
         // start of run x of the destination (x <= K), destination-local
         auto st = [&](int x) -> int64_t {
             return x >= K ? c.B.n : J.arc_cand_off[c.B.a0 + x - J.arc_base] - c.B.c0;
@@ -179,8 +181,9 @@ __global__ void __launch_bounds__(FilterCfg<T>::kThreads) big_lex_filter_kernel(
         const ExpandJob &J = jobs[W.job];
         BigItem B;
         if (!J.lex_big || !big_item_any(J, W, pass, &B) || !lex_eligible(J, B)) continue;
-        // sorted candidates: big_pts after an even number of merge rounds, else big_pts2
-        const T *cand = static_cast<const T *>(lex_merge_rounds(B.a1 - B.a0) & 1 ? J.big_pts2 : J.big_pts) + B.soff * 3;
+        // sorted candidates: big_pts after an even number of merge rounds, else the slab
+        const T *cand = lex_merge_rounds(B.a1 - B.a0) & 1 ? reinterpret_cast<const T *>(big_slab<3, T>(J, B.soff))
+                                                          : static_cast<const T *>(J.big_pts) + B.soff * 3;
         T *out = static_cast<T *>(J.out_pts) + B.c0 * 3;
         StairState st;
         int64_t kept = 0;

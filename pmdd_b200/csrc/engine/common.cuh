@@ -98,13 +98,11 @@ struct ExpandJob {
     int32_t *tile_first;           // [num_tiles+1]: first destination of each tile (tile_plan_kernel)
     const int64_t *big_list;       // (local item, scratch offset) pairs
     int32_t num_big;
-    int32_t pivot_rule;            // pivots per mark-path destination of n candidates:
-                                   // 1: 4*sqrt(n) within [32, 4096]; 0: n/64 within [512, 4096]
     void *big_pts;                 // scratch: candidates of oversized destinations (AoS)
-    void *big_pts2;                // scratch: the same candidates in sum-bucket order
-    void *big_surv;                // scratch: survivors of one bucket that overflow shared memory
-    int32_t *big_idx;              // scratch: candidate index of each bucket-ordered point
-    int32_t *big_surv_idx;         // scratch: candidate index of each overflowing survivor
+    void *big_slab;                // scratch: room for two more points per candidate, laid out per
+                                   // destination (big_common.cuh: big_slab)
+    int32_t *big_idx;              // scratch: an int per candidate (SFS index, mark-path key)
+    int32_t *big_surv_idx;         // scratch: another (SFS survivor index, place in the key's bucket)
     int64_t big_mark_min;          // oversized destinations of at least this many candidates take the mark path
     int64_t big_window;            // pass p takes the destinations whose scratch offset is in
                                    // [p * big_window, (p + 1) * big_window) (--max-cand)

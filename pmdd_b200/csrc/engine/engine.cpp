@@ -601,8 +601,6 @@ Engine::Engine(int device, int64_t budget_bytes, int max_slots, int stream_prior
     if (lb && *lb) lex_bulk_ = lb[0] == '1';
     const char *cl = std::getenv("PMDD_CHAIN_LAYERS");
     if (cl && *cl) chain_layers_ = std::max(0, std::min(std::atoi(cl), kChainMaxLayers));
-    const char *pr = std::getenv("PMDD_PIVOT_RULE");
-    if (pr && *pr) pivot_rule_ = std::strcmp(pr, "n64") == 0 ? 0 : 1;
     const char *cg = std::getenv("PMDD_CHAIN_GROW");
     if (cg && *cg) chain_grow_all_ = std::strcmp(cg, "all") == 0;
     const char *cr = std::getenv("PMDD_CHAIN_MAX_REQUESTS");
@@ -1197,6 +1195,11 @@ int Engine::step() {
         int64_t big_passes;        // scratch passes of the oversized path
         int64_t big_rows;          // oversized candidate rows over the group's jobs (flat space)
         int64_t mark_cap;          // upper bound on the group's mark-path destinations per pass
+        int64_t mark_min;          // largest crossover of its jobs
+    };
+    // SFS blocks: destinations that leave the tiles for their arc count, or below a raised crossover
+    auto with_sfs = [](const GroupLaunch &g) {
+        return g.mark_min > dev::kSmallMax + 1 || g.max_big_arcs > dev::kTileArcCap / 2;
     };
     std::vector<GroupLaunch> glaunch;
     std::vector<int64_t> tile_bases(exps.size()), item_bases(exps.size());  // group-relative
@@ -1206,7 +1209,7 @@ int Engine::step() {
         std::vector<ExpPlan> ordered;
         ordered.reserve(exps.size());
         for (auto &g : groups) {
-            GroupLaunch gl{g.first.first, g.first.second, pos, g.second.size(), 0, bigwork.size(), 0, 0, 0, 0, 0, 0, 0};
+            GroupLaunch gl{g.first.first, g.first.second, pos, g.second.size(), 0, bigwork.size(), 0, 0, 0, 0, 0, 0, 0, 0};
             for (size_t idx : g.second) {
                 const ExpPlan &e = exps[idx];
                 Instance &I = *e.I;
@@ -1257,15 +1260,15 @@ int Engine::step() {
                     const size_t ib = align256(sizeof(int32_t) * static_cast<size_t>(e.big_rows));
                     char *m = static_cast<char *>(e.big_mem);
                     J.big_pts = m;
-                    J.big_pts2 = m + pb;
-                    J.big_surv = m + 2 * pb;
+                    J.big_slab = m + pb;
                     J.big_idx = reinterpret_cast<int32_t *>(m + 3 * pb);
                     J.big_surv_idx = reinterpret_cast<int32_t *>(m + 3 * pb + ib);
                     J.big_window = e.big_window;
                     J.big_rows = e.big_rows;
-                    const int64_t mm = mark_min_for(I.d, I.opts.problem_type);
+                    // (the mark path's slab layout needs more than kSmallMax candidates)
+                    const int64_t mm = std::max<int64_t>(mark_min_for(I.d, I.opts.problem_type), dev::kSmallMax + 1);
                     J.big_mark_min = mm;
-                    J.pivot_rule = pivot_rule_;
+                    gl.mark_min = std::max(gl.mark_min, mm);
                     if (s.res.max_item >= mm) gl.mark_cap += e.big_rows / mm + 1;
                     gl.big_passes = std::max<int64_t>(gl.big_passes, (e.big_total + e.big_window - 1) / e.big_window);
                 }
@@ -1613,7 +1616,7 @@ int Engine::step() {
             const GroupLaunch &gl = glaunch[g];
             if (gl.big_count == 0) continue;
             const int64_t nw = static_cast<int64_t>(gl.big_count);
-            if (nw > sms_ * 3 && nw <= dev::kBigOrderMax) {
+            if (with_sfs(gl) && nw > sms_ * 3 && nw <= dev::kBigOrderMax) {
                 big_order[g] = static_cast<int32_t *>(scratch(sizeof(int32_t) * static_cast<size_t>(nw)));
                 if (!big_order[g]) count_alloc_ok = false;
             }
@@ -1924,7 +1927,7 @@ int Engine::step() {
         L.num_jobs = static_cast<int>(gl.count);
         L.total = gl.big_rows;
         L.sms = sms_;
-        L.with_sfs = true;
+        L.with_sfs = with_sfs(gl);
         L.lex_big = gl.d == 3 && lex_tiles_;
         L.lex_rounds = L.lex_big ? dev::lex_merge_rounds(std::min(gl.max_big_arcs, lex_max_arcs_)) : 0;
         L.mark_cap = static_cast<int>(std::min<int64_t>(gl.mark_cap, static_cast<int64_t>(gl.big_count)));
@@ -1936,7 +1939,8 @@ int Engine::step() {
         for (int64_t pass = 0; pass < gl.big_passes; ++pass) {
             L.pass = pass;
             if (!cuda_ok(dev::launch_big(gl.d, gl.wide, L, stream_), "oversized-destination kernels")) return -1;
-            launches_ += (L.mark_cap > 0 ? 9 : 2) + (ordered ? 1 : 0) + (L.lex_big ? 1 + L.lex_rounds : 0);
+            launches_ += 1 + (L.mark_cap > 0 ? 1 + dev::kMaximaLaunches : 0) + (L.with_sfs ? 1 + (ordered ? 1 : 0) : 0) +
+                         (L.lex_big ? 1 + L.lex_rounds : 0);
         }
     }
     if (!sdjobs.empty()) {

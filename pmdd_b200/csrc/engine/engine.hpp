@@ -361,9 +361,6 @@ class Engine {
     static constexpr int32_t kChainMaxLayers = 64;
     bool chain_grow_all_ = false;
     int64_t chain_max_requests_ = 128;
-    // Pivots of a mark-path destination of n candidates (big.cu): about 4*sqrt(n) (1), or
-    // n/64 with a floor of 512 (0, PMDD_PIVOT_RULE=n64).
-    int32_t pivot_rule_ = 1;
     int64_t chain_max_cand_ = int64_t(1) << 17;
     int64_t chained_layers_total_ = 0;  // layers expanded by chained steps (statistics)
     int32_t lex_max_arcs_ = kDefaultLexMaxArcs;

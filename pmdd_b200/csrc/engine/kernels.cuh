@@ -47,6 +47,7 @@ struct BigLaunch {
 // Most oversized destinations whose SFS blocks are put in size order (one block sorts them).
 constexpr int kBigOrderMax = 4096;
 size_t big_plan_bytes(int cap);
+constexpr int kMaximaLaunches = 6;  // kernels of one pass over a set of point sets (maxima.cuh)
 cudaError_t launch_big(int d, bool wide, const BigLaunch &L, cudaStream_t stream);
 // The lexicographic oversized path (big_lex.cu), three objectives: the rank kernel takes
 // the place of the materialising expansion, the filter runs after the other paths.
