@@ -444,7 +444,7 @@ int pmdd_pareto_filter(const int32_t *points, int64_t num_points, int32_t nobjs,
         if (e == cudaSuccess)
             e = pmdd::dev::launch_pareto_filter(nobjs, static_cast<const int32_t *>(d_in), num_points, d_scratch,
                                                 static_cast<int32_t *>(d_out), static_cast<int64_t *>(d_n), st);
-        E.count_launches(1);
+        E.count_launches(pmdd::dev::pareto_launches(num_points));
         int64_t n_out = 0;
         if (e == cudaSuccess) e = cudaMemcpyAsync(&n_out, d_n, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);

@@ -80,7 +80,7 @@ struct SegHead {
 template <typename T>
 struct Seg {
     const T *pts;                     // n points, D values each
-    int64_t n;                        // 1024 < n < 2^32
+    int64_t n;                        // 0 < n < 2^32
     unsigned char *slab;
     uint32_t *key;                    // [n]
     uint32_t *place;                  // [n] place within the key's bucket
