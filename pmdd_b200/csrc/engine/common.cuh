@@ -70,7 +70,6 @@ constexpr int kBigJTile = 1024;       // candidates per shared-memory comparison
 // Device error word bits (written with atomicOr; read back once per step).
 constexpr uint32_t kErrBounds = 1u;        // an index check failed (work skipped)
 constexpr uint32_t kErrCoupleOverflow = 2u;
-constexpr uint32_t kErrTimeout = 4u;       // a bounded wait (bulk-copy barrier) gave up
 
 // One layer expansion of one instance in one direction.  "Items" are the destination
 // nodes of the layer; each has a contiguous range of arcs whose neighbour (the arc's
@@ -119,7 +118,6 @@ struct ExpandJob {
     int32_t pair_max;              // lexicographic tiles: destinations of at most this many
                                    // candidates are checked pairwise, larger ones by a staircase warp
     int32_t lex_big;               // 1: oversized destinations with sorted runs take big_lex.cu
-    int32_t lex_bulk;              // 1: lexicographic tiles stage parent runs by bulk copies
     int32_t lex_max_arcs;          // oversized destinations of at most this many runs (and at
                                    // most kBigLexMaxArcs) take big_lex.cu
     unsigned long long *phase_clk; // diagnostic: cycles per tile phase (lexicographic tiles), or nullptr

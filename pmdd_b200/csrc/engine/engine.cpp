@@ -595,10 +595,6 @@ Engine::Engine(int device, int64_t budget_bytes, int max_slots, int stream_prior
     *(static_cast<unsigned char *>(h_init_.p) + kSeedTemplate + 76) = 1;
     const char *lx = std::getenv("PMDD_LEX_TILES");
     if (lx && lx[0] == '0') lex_tiles_ = false;
-    const char *sx = std::getenv("PMDD_SUM_TILES");
-    if (sx && *sx) sum_tiles_ = sx[0] == '1';
-    const char *lb = std::getenv("PMDD_LEX_BULK");
-    if (lb && *lb) lex_bulk_ = lb[0] == '1';
     const char *cl = std::getenv("PMDD_CHAIN_LAYERS");
     if (cl && *cl) chain_layers_ = std::max(0, std::min(std::atoi(cl), kChainMaxLayers));
     const char *cg = std::getenv("PMDD_CHAIN_GROW");
@@ -1246,7 +1242,6 @@ int Engine::step() {
                 J.out_sorted = e.out_sorted;
                 J.pair_max = pair_max_for(I.d, I.opts.problem_type);
                 J.lex_big = (I.d == 3 && lex_tiles_) ? 1 : 0;
-                J.lex_bulk = lex_bulk_ ? 1 : 0;
                 J.lex_max_arcs = lex_max_arcs_;
                 J.tile_base = gl.tiles;
                 tile_bases[pos] = gl.tiles;
@@ -1373,7 +1368,7 @@ int Engine::step() {
     const size_t f_sd = f_ts + 2 * sizeof(unsigned long long) * exps.size();  // (survivors, staircase) per expansion
     const size_t f_err = f_sd + sizeof(int64_t) * sdjobs.size();
     const size_t f_clk = f_err + sizeof(uint64_t);  // PMDD_TRACE: tile phase cycles (8 counters)
-    const size_t f_q = f_clk + (trace_ ? 10 * sizeof(unsigned long long) : 0);  // tile queue per group
+    const size_t f_q = f_clk + (trace_ ? 8 * sizeof(unsigned long long) : 0);  // tile queue per group
     const size_t f_total = f_q + sizeof(unsigned long long) * glaunch.size();
     char *d_fixed = static_cast<char *>(scratch(f_total));
     dev::CountResult *d_results = counts.empty() ? nullptr : reinterpret_cast<dev::CountResult *>(d_fixed);
@@ -1762,7 +1757,6 @@ int Engine::step() {
                 J.big_list = j == 1 ? new_big[c.count_idx] : c.big[pb];
                 J.pair_max = pair_max_for(I.d, I.opts.problem_type);
                 J.lex_big = (I.d == 3 && lex_tiles_) ? 1 : 0;
-                J.lex_bulk = lex_bulk_ ? 1 : 0;
                 J.lex_max_arcs = lex_max_arcs_;
                 g.items[j] += J.num_items;
                 g.tiles[j] += c.ntiles;
@@ -1904,9 +1898,9 @@ int Engine::step() {
         // blocks beyond the tiles would only be scheduled to exit (several waves of them at
         // the tiles' shared-memory size cost more than a small step's work)
         const int grid = static_cast<int>(std::min<int64_t>(sms_ * 8, std::max<int64_t>(1, gl.tiles)));
-        const bool lex = lex_tiles_for(gl.d, gl.wide);
+        const bool lex = lex_tiles_for(gl.d);
         const cudaError_t te =
-            lex ? dev::launch_expand_tiles_lex(gl.d, gl.wide, dj, dtb, static_cast<int>(gl.count), gl.tiles, grid, queue,
+            lex ? dev::launch_expand_tiles_lex(gl.wide, dj, dtb, static_cast<int>(gl.count), gl.tiles, grid, queue,
                                                nullptr, stream_)
                 : dev::launch_expand_tiles(gl.d, gl.wide, dj, dtb, static_cast<int>(gl.count), gl.tiles, grid, queue,
                                            nullptr, stream_);
@@ -2039,11 +2033,11 @@ int Engine::step() {
                         return -1;
                     launches_ += 2;
                 }
-                const bool lex = lex_tiles_for(g.d, g.wide);
+                const bool lex = lex_tiles_for(g.d);
                 // the tiles' bound assumes full buffers: one wave of blocks loops over them
                 const int grid = static_cast<int>(std::min<int64_t>(sms_ * 2, std::max<int64_t>(1, g.tiles[j])));
                 const cudaError_t te =
-                    lex ? dev::launch_expand_tiles_lex(g.d, g.wide, dj, dtb, static_cast<int>(n), g.tiles[j], grid, queue,
+                    lex ? dev::launch_expand_tiles_lex(g.wide, dj, dtb, static_cast<int>(n), g.tiles[j], grid, queue,
                                                        tiles_dev, stream_)
                         : dev::launch_expand_tiles(g.d, g.wide, dj, dtb, static_cast<int>(n), g.tiles[j], grid, queue,
                                                    tiles_dev, stream_);
@@ -2112,15 +2106,14 @@ int Engine::step() {
                      "[pmdd step] jobs=%zu counts=%zu couple=%zu cand=%lld big_items=%lld big_cand=%lld max_item=%lld "
                      "tile_cand=%lld tile_surv=%llu tiles=%lld tiles_ms=%.3f big_ms=%.3f rest_ms=%.3f host_to_sync_us=%.1f "
                      "plan_us=%.1f plan_exp_us=%.1f enqueue_us=%.1f release_us=%.1f wait_us=%.1f prev_post_us=%.1f "
-                     "arena_reserved_mb=%.0f arena_grow_ms=%.1f phase_mcyc=%.2f,%.2f,%.2f,%.2f,%.2f,%.2f,%.2f warp_mcyc=%.2f,%.2f\n",
+                     "arena_reserved_mb=%.0f arena_grow_ms=%.1f phase_mcyc=%.2f,%.2f,%.2f,%.2f,%.2f,%.2f,%.2f\n",
                      exps.size(), counts.size(), ujobs.size(), static_cast<long long>(cand),
                      static_cast<long long>(nbig), static_cast<long long>(big_cand), static_cast<long long>(max_item),
                      static_cast<long long>(cand - big_cand), tile_surv, step_tiles, ms_expand, ms_big, ms_rest,
                      (now_s() - step_t0) * 1e6, (t_issue - step_t0) * 1e6, (t_p1 - step_t0) * 1e6,
                      (t_rel - t_issue) * 1e6, (t_enq - t_rel) * 1e6, (t_sync - t_enq) * 1e6, last_post_us_,
                      arena_.reserved() / 1e6, arena_.grow_seconds() * 1e3,
-                     pc[0] * 1e-6, pc[1] * 1e-6, pc[2] * 1e-6, pc[3] * 1e-6, pc[4] * 1e-6, pc[5] * 1e-6, pc[6] * 1e-6,
-                     pc[7] * 1e-6, pc[8] * 1e-6);
+                     pc[0] * 1e-6, pc[1] * 1e-6, pc[2] * 1e-6, pc[3] * 1e-6, pc[4] * 1e-6, pc[5] * 1e-6, pc[6] * 1e-6);
     }
     for (void *q : step_scratch_) arena_.release(q);
     step_scratch_.clear();
@@ -2128,12 +2121,8 @@ int Engine::step() {
     // ----------------------------------------------------------- host updates
     const uint32_t errw = *reinterpret_cast<uint32_t *>(hsum + s_err);
     if (errw != 0) {
-        const bool timeout = (errw & dev::kErrTimeout) != 0 && (errw & ~dev::kErrTimeout) == 0;
         for (auto &p : active_)
-            if (p->phase != Instance::DONE) {
-                if (timeout) fail(*p, PMDD_ERR_TIMEOUT, "a bounded device wait gave up (bulk-copy staging)");
-                else fail(*p, PMDD_ERR_INTERNAL, "device-side index check failed");
-            }
+            if (p->phase != Instance::DONE) fail(*p, PMDD_ERR_INTERNAL, "device-side index check failed");
     }
     for (size_t k = 0; k < exps.size(); ++k) {
         const ExpPlan &e = exps[k];

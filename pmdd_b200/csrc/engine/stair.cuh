@@ -10,8 +10,7 @@
 // survivors are checked against each other (an earlier one dominates; a later one that
 // is at least as large in both objectives and differs removes an entry from the next
 // staircase), and the next staircase is the surviving entries merged with the chunk's
-// new maxima.  Used by the tile kernel (tile_lex.cu) and the oversized-destination path
-// (big_lex.cu).
+// new maxima.  Used by the oversized-destination path (big_lex.cu).
 #pragma once
 
 #include <cstdint>
