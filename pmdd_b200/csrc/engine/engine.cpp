@@ -791,8 +791,8 @@ void Engine::release_instance(Instance &I) {
     arena_.release(I.cu_mem);
     arena_.release(I.cu_ctr);
     I.dd = nullptr;
-    I.cu_mem = I.cu_U = I.cu_U_alt = I.cu_p2 = I.cu_sv = nullptr;
-    I.cu_i2 = I.cu_si = I.cu_hist = nullptr;
+    I.cu_mem = I.cu_U = I.cu_U_alt = I.cu_slab = nullptr;
+    I.cu_i2 = I.cu_si = nullptr;
     I.cu_ctr = nullptr;
     I.blob.clear();
     I.blob.shrink_to_fit();
@@ -836,11 +836,9 @@ bool Engine::carve_couple(Instance &I, int64_t ucap) {
     I.cu_mem = mem;
     I.cu_U = m;
     I.cu_U_alt = m + pts;
-    I.cu_p2 = m + 2 * pts;
-    I.cu_sv = m + 3 * pts;
+    I.cu_slab = m + 2 * pts;
     I.cu_i2 = reinterpret_cast<int32_t *>(m + 4 * pts);
     I.cu_si = reinterpret_cast<int32_t *>(m + 4 * pts + idx);
-    I.cu_hist = reinterpret_cast<int32_t *>(m + 4 * pts + 2 * idx);
     if (old_U && I.result_n > 0)  // carry the running frontier over (growth)
         cudaMemcpyAsync(I.cu_U, old_U, static_cast<size_t>(I.result_n) * I.d * I.elem(), cudaMemcpyDeviceToDevice,
                         stream_);
@@ -1831,7 +1829,8 @@ int Engine::step() {
         I->stats.cutset_size = I->nodes_in(I->td.layer);
         // running frontier + one round of survivors; the seed round needs d+1 per node
         const int64_t ucap = std::max<int64_t>(1 << 17, static_cast<int64_t>(I->stats.cutset_size) * (I->d + 1) + 4096);
-        I->cu_ctr = static_cast<int64_t *>(arena_.alloc(sizeof(int64_t) * dev::kCtrCount));
+        I->cu_ctr = static_cast<int64_t *>(
+            arena_.alloc(sizeof(int64_t) * (dev::kCtrCount + static_cast<size_t>(I->stats.cutset_size) + 1)));
         if (!I->cu_ctr || !carve_couple(*I, ucap)) {
             fail(*I, PMDD_ERR_OOM, "device memory budget exhausted at the cutset join");
             continue;
@@ -1855,18 +1854,16 @@ int Engine::step() {
         J.U = I->cu_U;
         J.U_alt = I->cu_U_alt;
         J.ucap = I->cu_ucap;
-        J.sc_pts2 = I->cu_p2;
-        J.sc_surv = I->cu_sv;
+        J.sc_slab = I->cu_slab;
         J.sc_idx = I->cu_i2;
         J.sc_sidx = I->cu_si;
-        J.sc_hist = I->cu_hist;
         J.ctr = I->cu_ctr;
         // the next running frontier lands in U_alt: swap now (host view)
         std::swap(I->cu_U, I->cu_U_alt);
         const bool is_new = std::find(entering.begin(), entering.end(), I) != entering.end();
         int64_t *ci = reinterpret_cast<int64_t *>(hs + off_ctrinit) + dev::kCtrCount * ujobs.size();
         std::memset(ci, 0, sizeof(int64_t) * dev::kCtrCount);
-        ci[dev::kCtrResume] = J.num_nodes;
+        ci[dev::kCtrResume] = INT64_MAX;
         ci[dev::kCtrValidEnd] = J.ucap;
         ujobs.push_back(J);
         ujob_inst.push_back(I);
@@ -1962,12 +1959,6 @@ int Engine::step() {
         for (size_t k = 0; k < ujobs.size(); ++k)
             ug[std::make_tuple(ujob_inst[k]->d, ujob_inst[k]->wide, ujob_inst[k]->couple_rounds == 0)].push_back(k);
         const dev::CoupleJob *du = reinterpret_cast<const dev::CoupleJob *>(d_stage + off_u);
-        // new requests: product statistics once
-        for (size_t k = 0; k < ujobs.size(); ++k) {
-            if (!ujob_new[k]) continue;
-            dev::launch_couple_products(du + k, 1, stream_);
-            launches_ += 1;
-        }
         for (auto &g : ug) {
             // jobs of one group are contiguous only if sorted; launch per job run
             size_t i = 0;
@@ -1977,11 +1968,19 @@ int Engine::step() {
                 const int n = static_cast<int>(j - i + 1);
                 // three 256-thread blocks per SM: the prune kernel's register limit
                 const int per = std::max(1, (sms_ * 3) / n);
+                const bool seed = std::get<2>(g.first);
+                int64_t points = 1;  // a seed round appends d + 1 points per cutset node
+                for (size_t k = i; k <= j; ++k)
+                    points = std::max<int64_t>(points, seed ? std::min<int64_t>(ujobs[g.second[k]].ucap,
+                                                                                int64_t(ujobs[g.second[k]].num_nodes) *
+                                                                                    (std::get<0>(g.first) + 1))
+                                                            : ujobs[g.second[k]].ucap);
+                int64_t nl = 0;
                 if (!cuda_ok(dev::launch_couple_round(std::get<0>(g.first), std::get<1>(g.first), du + g.second[i], n,
-                                                      per, std::get<2>(g.first), stream_),
+                                                      per, seed, points, &nl, stream_),
                              "coupling round"))
                     return -1;
-                launches_ += 7;
+                launches_ += nl;
                 i = j + 1;
             }
         }

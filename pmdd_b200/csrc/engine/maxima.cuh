@@ -80,12 +80,12 @@ struct SegHead {
 template <typename T>
 struct Seg {
     const T *pts;                     // n points, D values each
-    int64_t n;                        // 0 < n < 2^32
+    int64_t n;                        // < 2^32
     unsigned char *slab;
     uint32_t *key;                    // [n]
     uint32_t *place;                  // [n] place within the key's bucket
     T *out;                           // survivors, D values each
-    int32_t *out_size;
+    int32_t *out_size;                // their number (nullptr with ordered output)
 };
 
 template <int D, typename T>
@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(kMaxStatThreads) maxima_stats_kernel(Src src) 
     src.template seg<D>(h, &g);
     const SegView<D, T> v = seg_view<D, T>(g.slab, g.n);
     const int m = g.n < kMaxSample ? static_cast<int>(g.n) : kMaxSample;
+    if (m <= 0) return;  // an empty segment (ordered output only): no chunks either
     if (tid < D) {
         s_mn[tid] = g.pts[tid];
         s_mx[tid] = g.pts[tid];
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(kMaxStatThreads) maxima_stats_kernel(Src src) 
         s_smax = 0;
         s_smin = ~0ull;
         s_npiv = 0;
-        *g.out_size = 0;
+        if (g.out_size) *g.out_size = 0;
     }
     for (int k = tid; k < D * kMaxBins; k += kMaxStatThreads) s_hist[k] = 0;
     for (int k = tid; k < SB; k += kMaxStatThreads) s_sum[k] = 0;
@@ -465,6 +466,7 @@ __global__ void __launch_bounds__(kMaxStatThreads) maxima_scan_kernel(Src src) {
     if (h >= src.count()) return;
     Seg<T> g;
     src.template seg<D>(h, &g);
+    if (g.n <= 0) return;
     const SegView<D, T> v = seg_view<D, T>(g.slab, g.n);
     const int64_t nb = int64_t(1) << v.bits;
     uint32_t carry = 0;
@@ -530,7 +532,7 @@ __global__ void __launch_bounds__(kMaxThreads) maxima_corner_kernel(Src src) {
     for (int o = 0; o < D; ++o) v.corner[o * v.groups + t] = mx[o];
 }
 
-template <int D, typename T, class Src>
+template <int D, typename T, bool ORDERED, class Src>
 __global__ void __launch_bounds__(kMaxThreads) maxima_mark_kernel(Src src) {
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -604,11 +606,18 @@ __global__ void __launch_bounds__(kMaxThreads) maxima_mark_kernel(Src src) {
         }
         const unsigned now = __ballot_sync(kAll, dom);
         if (now != dead) {
-            if (now == kAll) return;
+            if (now == kAll) {
+                if (ORDERED && lane == 0) g.place[w0 >> 5] = 0;
+                return;
+            }
             dead = now;
 #pragma unroll
             for (int o = 0; o < D; ++o) lo[o] = warp_min_of<T>(p[o]);
         }
+    }
+    if (ORDERED) {  // maxima_order_kernel and maxima_write_kernel follow
+        if (lane == 0) g.place[w0 >> 5] = ~dead;
+        return;
     }
     int32_t at = 0;
     if (lane == 0) at = atomicAdd(g.out_size, __popc(~dead));
@@ -620,8 +629,52 @@ __global__ void __launch_bounds__(kMaxThreads) maxima_mark_kernel(Src src) {
     }
 }
 
-// `segs`: upper bound on the segments, `chunks`: on their 256-point chunks.
+// Ordered output, block per segment: survivors before each 32 rows (into key), and their
+// number to src.finish.
 template <int D, typename T, class Src>
+__global__ void __launch_bounds__(kMaxStatThreads) maxima_order_kernel(Src src) {
+    __shared__ int64_t warp_buf[32];
+    __shared__ int64_t s_total;
+    const int h = blockIdx.x;
+    if (h >= src.count()) return;
+    Seg<T> g;
+    src.template seg<D>(h, &g);
+    int64_t carry = 0;
+    if (g.n > 0) {
+        const int64_t warps = (static_cast<int64_t>(seg_view<D, T>(g.slab, g.n).head->rows) + 31) / 32;
+        for (int64_t w0 = 0; w0 < warps; w0 += kMaxStatThreads) {
+            const int64_t w = w0 + threadIdx.x;
+            const int64_t c = w < warps ? __popc(g.place[w]) : 0;
+            const int64_t ex = block_exclusive_scan<int64_t, kMaxStatThreads>(c, warp_buf, &s_total);
+            if (w < warps) g.key[w] = static_cast<uint32_t>(carry + ex);
+            carry += s_total;
+        }
+    }
+    if (threadIdx.x == 0) src.finish(h, carry);
+}
+
+// Ordered output: the survivors in row order.
+template <int D, typename T, class Src>
+__global__ void __launch_bounds__(kMaxThreads) maxima_write_kernel(Src src) {
+    int h;
+    int64_t base;
+    if (!src.chunk(blockIdx.x, &h, &base)) return;
+    Seg<T> g;
+    src.template seg<D>(h, &g);
+    const SegView<D, T> v = seg_view<D, T>(g.slab, g.n);
+    const int64_t i = base + threadIdx.x;
+    if (i >= v.head->rows) return;
+    const unsigned keep = g.place[i >> 5], lane = threadIdx.x & 31;
+    if (((keep >> lane) & 1u) == 0) return;
+    const SortedPt<D, T> q = v.rows[i];
+    T *out = g.out + (static_cast<int64_t>(g.key[i >> 5]) + __popc(keep & ((1u << lane) - 1u))) * D;
+#pragma unroll
+    for (int o = 0; o < D; ++o) out[o] = q.v[o];
+}
+
+// `segs`: upper bound on the segments, `chunks`: on their 256-point chunks.
+// ORDERED: survivors in the rows' order, their number to src.finish(segment, number).
+template <int D, typename T, bool ORDERED = false, class Src>
 cudaError_t launch_maxima(const Src &src, int segs, int64_t chunks, cudaStream_t stream) {
     const unsigned c = static_cast<unsigned>(chunks);
     maxima_stats_kernel<D, T, Src><<<segs, kMaxStatThreads, 0, stream>>>(src);
@@ -629,7 +682,11 @@ cudaError_t launch_maxima(const Src &src, int segs, int64_t chunks, cudaStream_t
     maxima_scan_kernel<D, T, Src><<<segs, kMaxStatThreads, 0, stream>>>(src);
     maxima_scatter_kernel<D, T, Src><<<c, kMaxThreads, 0, stream>>>(src);
     maxima_corner_kernel<D, T, Src><<<(c + kMaxThreads / 32 - 1) / (kMaxThreads / 32), kMaxThreads, 0, stream>>>(src);
-    maxima_mark_kernel<D, T, Src><<<c, kMaxThreads, 0, stream>>>(src);
+    maxima_mark_kernel<D, T, ORDERED, Src><<<c, kMaxThreads, 0, stream>>>(src);  // kMaximaLaunches kernels
+    if constexpr (ORDERED) {
+        maxima_order_kernel<D, T, Src><<<segs, kMaxStatThreads, 0, stream>>>(src);
+        maxima_write_kernel<D, T, Src><<<c, kMaxThreads, 0, stream>>>(src);
+    }
     return cudaGetLastError();
 }
 
