@@ -34,13 +34,11 @@ inline cudaError_t ensure_smem_limit(const void *func, size_t bytes) {
 // global-memory ("big") path.  A tile therefore holds < 2*kTileWindow candidates.  The
 // window shrinks (to kTileWindowMin) for steps with few candidates, so that a small
 // step still spreads over the SMs.
-constexpr int kTileThreads = 512;
 constexpr int kTileWindow = 1024;
 constexpr int kTileWindowMin = 128;
 constexpr int kSmallMax = 1024;
 constexpr int kTileCap = 2 * kTileWindow;
-// Per-pass staging caps, sized so that a tile's shared memory (about 70 KB at d=3) lets
-// three 512-thread blocks share an SM.
+// Per-pass staging caps.
 constexpr int kTileItemCap = 512;    // destinations staged per pass inside one tile
 constexpr int kTileArcCap = 1024;    // arcs staged per pass inside one tile
 

@@ -1,4 +1,4 @@
-"""The three-objective tile kernel (tile_lex.cu) where its chunks can go wrong: small
+"""The three-objective tile kernel (lex_items.cuh) where its chunks can go wrong: small
 objective ranges (equal values of objective 1 and equal points inside a chunk and across
 chunks), antichains in objectives 1 and 2 (full staircases), and int64 points."""
 from __future__ import annotations
