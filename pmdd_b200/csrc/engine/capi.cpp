@@ -562,6 +562,7 @@ int pmdd_resident_enumerate(pmdd_resident *R, const pmdd_options *opts, pmdd_fro
         I->blob_bytes = T.blob_bytes;
         I->dev_bytes = T.dev_bytes;
         I->dd = T.dd;
+        I->d_layer_off = T.d_layer_off;
         I->d_in_off = T.d_in_off;
         I->d_arc_src = T.d_arc_src;
         I->d_arc_w = T.d_arc_w;

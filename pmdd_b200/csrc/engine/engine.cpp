@@ -597,6 +597,8 @@ Engine::Engine(int device, int64_t budget_bytes, int max_slots, int stream_prior
     if (lx && lx[0] == '0') lex_tiles_ = false;
     const char *cl = std::getenv("PMDD_CHAIN_LAYERS");
     if (cl && *cl) chain_layers_ = std::max(0, std::min(std::atoi(cl), kChainMaxLayers));
+    const char *rl = std::getenv("PMDD_RUN_LAYERS");
+    if (rl && *rl) run_layers_ = std::max(0, std::atoi(rl));
     const char *cg = std::getenv("PMDD_CHAIN_GROW");
     if (cg && *cg) chain_grow_all_ = std::strcmp(cg, "all") == 0;
     const char *cr = std::getenv("PMDD_CHAIN_MAX_REQUESTS");
@@ -865,6 +867,7 @@ bool Engine::upload_dd(Instance &I) {
 bool Engine::bind_dd(Instance &I) {
     if (I.tsp) {  // shared structure: only the weight table is the instance's own
         const TspStructure &S = *I.tsp;
+        I.d_layer_off = reinterpret_cast<const int32_t *>(S.mem);  // the structure's first array
         I.d_in_off = S.in_off;
         I.d_arc_src = S.arc_src;
         I.d_arc_w = S.arc_w;
@@ -878,6 +881,7 @@ bool Engine::bind_dd(Instance &I) {
         I.d_cursor = S.cursor;
         return true;
     }
+    I.d_layer_off = reinterpret_cast<const int32_t *>(I.dd + I.off_layer);
     I.d_in_off = reinterpret_cast<const int32_t *>(I.dd + I.off_in);
     I.d_arc_src = reinterpret_cast<const int32_t *>(I.dd + I.off_src);
     I.d_arc_w = reinterpret_cast<const int32_t *>(I.dd + I.off_w);
@@ -1036,6 +1040,65 @@ struct ChainGroup {
 
 std::atomic<int64_t> g_total_launches{0};
 
+void Engine::release_run(RunSlot &r) {
+    for (char *&b : r.buf) {
+        arena_.release(b);
+        b = nullptr;
+    }
+    r.I->in_run = false;
+}
+
+void Engine::plan_runs(std::vector<RunSlot> &runs) {
+    for (auto &p : active_) p->in_run = false;
+    if (run_layers_ <= 0 || chain_layers_ <= 0 || static_cast<int64_t>(active_.size()) > kRunMaxRequests) return;
+    // other requests wait for the step's runs: long ones only when nothing else is under way
+    bool others = !queued_.empty();
+    std::vector<Instance *> picked;
+    for (auto &p : active_) {
+        Instance &I = *p;
+        if (I.phase == Instance::DONE) continue;
+        const Side &s = I.td;
+        const bool small = s.counted ? s.res.total <= kRunEnter && s.res.num_big == 0 : s.layer == 0;
+        bool ok = I.phase == Instance::RUNNING && I.opts.method == 1 && small && s.layer < I.L - 1;
+        if (ok && I.run_skip > 0) {  // its last run stopped at once: a few ordinary steps first
+            --I.run_skip;
+            ok = false;
+        }
+        if (ok) picked.push_back(&I);
+        else others = true;
+    }
+    for (Instance *p : picked) {
+        Instance &I = *p;
+        RunSlot r;
+        r.I = &I;
+        r.sd = I.opts.state_dominance > 0 && I.sd_kind != 0 && I.sd_kind == I.opts.problem_type && I.d_sd_order;
+        r.last = static_cast<int32_t>(std::min<int64_t>(
+            I.L - 1, static_cast<int64_t>(I.td.layer) + (others ? std::min(run_layers_, kRunShared) : run_layers_)));
+        for (int l = I.td.layer + 1; l <= r.last; ++l) {
+            r.vcap = std::max(r.vcap, I.nodes_in(l));
+            r.max_arcs = std::max(r.max_arcs, I.arc_at_layer[l + 1] - I.arc_at_layer[l]);
+        }
+        r.max_nodes = r.vcap;
+        if (r.last < I.L - 1) {
+            r.max_nodes = std::max(r.max_nodes, I.nodes_in(r.last + 1));
+            r.max_arcs = std::max(r.max_arcs, I.arc_at_layer[r.last + 2] - I.arc_at_layer[r.last + 1]);
+        }
+        r.vcap = static_cast<int32_t>(std::min<int64_t>(r.vcap, dev::kRunCap));
+        r.pts_at = align256(sizeof(int64_t) * r.vcap) + align256((sizeof(int32_t) + 1) * static_cast<size_t>(r.vcap));
+        const size_t bytes = r.pts_at + static_cast<size_t>(dev::kRunCap) * I.d * I.elem();
+        // two sets beside what is in use, with room to spare; else an ordinary step
+        if (arena_.used() + 4 * bytes > arena_.capacity()) continue;
+        r.buf[0] = static_cast<char *>(arena_.alloc(bytes));
+        r.buf[1] = r.buf[0] ? static_cast<char *>(arena_.alloc(bytes)) : nullptr;
+        if (!r.buf[1]) {
+            arena_.release(r.buf[0]);
+            continue;
+        }
+        I.in_run = true;
+        runs.push_back(r);
+    }
+}
+
 int Engine::step() {
     if (!ok_ || !make_current()) return -1;
     const double step_t0 = trace_ ? now_s() : 0.0;
@@ -1089,14 +1152,27 @@ int Engine::step() {
         counters_.admitted++;
         reserved += std::max<int64_t>(0, pred - current_bytes(I));
         if (I.phase == Instance::RUNNING) {
-            counts.push_back({&I, true, false});
-            if (I.opts.method == 3) counts.push_back({&I, false, false});
+            if (I.opts.method == 3) {
+                counts.push_back({&I, true, false});
+                counts.push_back({&I, false, false});
+            }  // method 1: a layer run from the root, or its count, below
         }
         active_.push_back(std::move(*it));
         it = queued_.erase(it);
     }
     counters_.running_peak = std::max<int64_t>(counters_.running_peak, static_cast<int64_t>(active_.size()));
     counters_.queued_peak = std::max<int64_t>(counters_.queued_peak, static_cast<int64_t>(queued_.size()));
+
+    // ------------------------------------------------------------ layer runs
+    // Requests by method 1 at the root, or whose next layer is small, run on from there in
+    // one launch (run.cu) instead of expanding one layer.
+    std::vector<RunSlot> runs;
+    plan_runs(runs);
+    for (auto &p : active_) {
+        Instance &I = *p;
+        if (I.phase == Instance::RUNNING && I.opts.method == 1 && I.td.layer == 0 && !I.td.counted && !I.in_run)
+            counts.push_back({&I, true, false});
+    }
 
     // ------------------------------------------------------------ expansions
     std::vector<ExpPlan> exps;
@@ -1107,7 +1183,7 @@ int Engine::step() {
     int64_t step_cand = 0;
     for (auto &p : active_) {
         const Instance &I = *p;
-        if (I.phase != Instance::RUNNING) continue;
+        if (I.phase != Instance::RUNNING || I.in_run) continue;
         const bool is_td = I.opts.method != 3 || I.td.score <= I.bu.score;
         const Side &s = is_td ? I.td : I.bu;
         if (s.counted) step_cand += s.res.total;
@@ -1117,7 +1193,7 @@ int Engine::step() {
                                                                                           step_cand / want_tiles));
     for (auto &p : active_) {
         Instance &I = *p;
-        if (I.phase != Instance::RUNNING) continue;
+        if (I.phase != Instance::RUNNING || I.in_run) continue;
         bool is_td = true;
         if (I.opts.method == 3) is_td = I.td.score <= I.bu.score;
         Side &s = is_td ? I.td : I.bu;
@@ -1355,6 +1431,12 @@ int Engine::step() {
             if (td_layer != bu_layer) counts.push_back({&I, e.td, true});
         }
     }
+    // a run's request is counted where the run stops (the kernel completes the job)
+    const size_t first_run_count = counts.size();
+    for (RunSlot &r : runs) {
+        r.count_idx = counts.size();
+        counts.push_back({r.I, true, false});
+    }
     std::vector<dev::CountJob> cjobs(counts.size());
     std::vector<int64_t *> new_arc_off(counts.size(), nullptr);
     std::vector<int64_t *> new_big(counts.size(), nullptr);
@@ -1420,6 +1502,25 @@ int Engine::step() {
     for (size_t k = 0; k < counts.size() && count_alloc_ok; ++k) {
         Instance &I = *counts[k].I;
         const bool td = counts[k].td;
+        if (k >= first_run_count) {  // sized for any layer the run may stop at
+            const RunSlot &r = runs[k - first_run_count];
+            dev::CountJob &J = cjobs[k];
+            std::memset(&J, 0, sizeof(J));
+            J.item_arc_off = I.d_in_off;
+            J.arc_nbr = I.d_arc_src;
+            const size_t arc_bytes = align256(sizeof(int64_t) * (static_cast<size_t>(r.max_arcs) + 1));
+            char *cb = static_cast<char *>(arena_.alloc(arc_bytes + sizeof(int64_t) * 2 * std::max(1, r.max_nodes)));
+            new_arc_off[k] = reinterpret_cast<int64_t *>(cb);
+            new_big[k] = cb ? reinterpret_cast<int64_t *>(cb + arc_bytes) : nullptr;
+            if (!cb) {
+                count_alloc_ok = false;
+                break;
+            }
+            J.arc_cand_off = new_arc_off[k];
+            J.big_list = new_big[k];
+            J.result = d_results + k;
+            continue;
+        }
         auto cur = side_after(I, td);
         const int l = cur.first;
         const int nl = td ? l + 1 : l - 1;
@@ -1585,6 +1686,24 @@ int Engine::step() {
         }
         if (chains.empty()) stage_bytes = align256(off_ctrinit + sizeof(int64_t) * dev::kCtrCount * n_couple_max);
     }
+    // layer runs: descriptors staged by (objectives, point type); per run what the host reads
+    // back (zeroed) and keep flags
+    std::sort(runs.begin(), runs.end(), [](const RunSlot &a, const RunSlot &b) {
+        return std::make_tuple(a.I->d, a.I->wide, a.count_idx) < std::make_tuple(b.I->d, b.I->wide, b.count_idx);
+    });
+    const size_t st_run = align256(stage_bytes);
+    if (!runs.empty()) stage_bytes = st_run + sizeof(dev::RunJob) * runs.size();
+    const size_t run_out_bytes = align256(sizeof(dev::RunOut) * runs.size());
+    char *d_run = nullptr;
+    if (!runs.empty() && count_alloc_ok) {
+        size_t bytes = run_out_bytes;
+        for (RunSlot &r : runs) {
+            r.at_keep = bytes;
+            if (r.sd) bytes += align256(static_cast<size_t>(dev::kRunCap));
+        }
+        d_run = static_cast<char *>(scratch(bytes));
+        if (d_run == nullptr) count_alloc_ok = false;
+    }
     // Every device and pinned allocation of the step is made here, before any side moves
     // or launch, so that running out of memory rolls the step back and fails one request
     // instead of the engine.
@@ -1597,7 +1716,8 @@ int Engine::step() {
     // ... | the chain block | the terminal sizes of chained requests
     const size_t s_chain = align256(s_fin + sizeof(int32_t) * exps.size());
     const size_t s_chfin = s_chain + chain_dev_bytes;
-    const size_t s_total = s_chfin + sizeof(int32_t) * chain_slots;
+    const size_t s_run = align256(s_chfin + sizeof(int32_t) * chain_slots);
+    const size_t s_total = s_run + run_out_bytes;
     // oversized path: per group, the size-order list and the mark-path plan
     std::vector<int32_t *> big_order(glaunch.size(), nullptr);
     std::vector<void *> big_plan(glaunch.size(), nullptr);
@@ -1632,6 +1752,7 @@ int Engine::step() {
                 arena_.release(q);
         }
         release_chains();
+        for (RunSlot &r : runs) release_run(r);
         for (void *q : step_scratch_) arena_.release(q);
         step_scratch_.clear();
         // the request with the largest expansion of this step (else the last one counted)
@@ -1671,6 +1792,44 @@ int Engine::step() {
     if (!sdjobs.empty()) {
         std::memcpy(hs + off_sd, sdjobs.data(), sizeof(dev::StateDomJob) * sdjobs.size());
         std::memcpy(hs + off_sdb, sd_bases.data(), sizeof(int64_t) * sd_bases.size());
+    }
+    for (size_t k = 0; k < runs.size(); ++k) {
+        const RunSlot &r = runs[k];
+        Instance &I = *r.I;
+        dev::RunJob J;
+        std::memset(&J, 0, sizeof(J));
+        J.item_arc_off = I.d_in_off;
+        J.arc_nbr = I.d_arc_src;
+        J.arc_wrow = I.d_arc_w;
+        J.weights = I.d_weights;
+        J.layer_off = I.d_layer_off;
+        J.pts = I.td.pts;
+        J.off = I.td.off;
+        J.size = I.td.size;
+        J.sorted = I.td.sorted;
+        J.layer = I.td.layer;
+        J.last = r.last;
+        J.terminal = I.L - 1;
+        for (int b = 0; b < 2; ++b) {
+            J.b_off[b] = reinterpret_cast<int64_t *>(r.buf[b]);
+            J.b_size[b] = r.size(b);
+            J.b_sorted[b] = r.sorted(b);
+            J.b_pts[b] = r.pts(b);
+        }
+        J.vcap = r.vcap;
+        J.pair_max = pair_max_for(I.d, I.opts.problem_type);
+        if (r.sd) {
+            J.sd_kind = I.sd_kind;
+            J.sd_order = I.d_sd_order;
+            J.sd_next = I.d_sd_next;
+            J.sd_state = I.d_state;
+            J.state_words = I.state_words;
+            J.keep = reinterpret_cast<uint8_t *>(d_run + r.at_keep);
+        }
+        J.out = reinterpret_cast<dev::RunOut *>(d_run) + k;
+        J.count = reinterpret_cast<dev::CountJob *>(d_stage + off_c) + r.count_idx;
+        J.err = d_err_step;
+        std::memcpy(hs + st_run + sizeof(dev::RunJob) * k, &J, sizeof(J));
     }
     // chained layers: every descriptor but the sizes the prep kernel fills in
     for (auto &g : chains) {
@@ -1905,6 +2064,21 @@ int Engine::step() {
         launches_ += 2;
         ktimes_.tile_launches += 1;
     }
+    if (!runs.empty()) {
+        cudaMemsetAsync(d_run, 0, run_out_bytes, stream_);
+        for (size_t i = 0; i < runs.size();) {
+            size_t j = i + 1;
+            while (j < runs.size() && runs[j].I->d == runs[i].I->d && runs[j].I->wide == runs[i].I->wide) ++j;
+            if (!cuda_ok(dev::launch_layer_runs(runs[i].I->d, runs[i].I->wide, lex_tiles_for(runs[i].I->d),
+                                                reinterpret_cast<const dev::RunJob *>(d_stage + st_run) + i,
+                                                static_cast<int>(j - i), stream_),
+                         "run_layers_kernel"))
+                return -1;
+            launches_ += 1;
+            ktimes_.tile_launches += 1;
+            i = j;
+        }
+    }
     cudaEventRecord(ev1, stream_);
     for (size_t g = 0; g < glaunch.size(); ++g) {
         const GroupLaunch &gl = glaunch[g];
@@ -2066,6 +2240,8 @@ int Engine::step() {
                                     sizeof(int32_t), cudaMemcpyDeviceToHost, stream_);
             }
     }
+    if (!runs.empty())
+        cudaMemcpyAsync(hsum + s_run, d_run, run_out_bytes, cudaMemcpyDeviceToHost, stream_);
     const double t_rel = trace_ ? now_s() : 0.0;
     for (void *q : to_release) arena_.release(q);
     const double t_enq = trace_ ? now_s() : 0.0;  // every copy and launch enqueued
@@ -2137,7 +2313,7 @@ int Engine::step() {
     for (size_t k = 0; k < sdjobs.size(); ++k)
         sd_inst[k]->stats.dominance_filtered_total += reinterpret_cast<const int64_t *>(hsum + s_sd)[k];
     const dev::CountResult *hres = reinterpret_cast<const dev::CountResult *>(hsum + s_counts);
-    for (size_t k = 0; k < counts.size(); ++k) {
+    for (size_t k = 0; k < first_run_count; ++k) {
         Instance &I = *counts[k].I;
         Side &s = counts[k].td ? I.td : I.bu;
         s.arc_off = new_arc_off[k];
@@ -2167,6 +2343,76 @@ int Engine::step() {
         I.stats.work_frontier_peak_points = std::max<int64_t>(I.stats.work_frontier_peak_points, n);
         I.phase = Instance::DONE;
     }
+    // requests that ran move to the layer they stopped at
+    int64_t run_layers = 0;
+    for (size_t k = 0; k < runs.size(); ++k) {
+        RunSlot &r = runs[k];
+        Instance &I = *r.I;
+        I.in_run = false;
+        const dev::RunOut &o = reinterpret_cast<const dev::RunOut *>(hsum + s_run)[k];
+        int64_t *arc_off = new_arc_off[r.count_idx], *big = new_big[r.count_idx];
+        if (I.phase != Instance::RUNNING) {  // cancelled or failed
+            release_run(r);
+            arena_.release(arc_off);
+            continue;
+        }
+        Side &s = I.td;
+        I.stats.kernel_expand_td_s += ms_expand * 1e-3;
+        I.stats.kernel_total_s += (ms_expand + ms_rest) * 1e-3;
+        run_layers += o.done;
+        I.run_skip = o.done == 0 ? kRunSkip : 0;
+        arena_.release(s.arc_off);
+        arena_.release(s.big_list);
+        s.arc_off = nullptr;
+        s.big_list = nullptr;
+        if (o.done > 0) {
+            I.stats.work_candidates_total += o.cand_total;
+            I.stats.work_candidates_peak = std::max(I.stats.work_candidates_peak, o.cand_peak);
+            I.peak_cand = std::max(I.peak_cand, o.cand_peak);
+            I.stats.work_tile_candidates_total += o.cand_total;
+            I.stats.work_tile_survivors_total += o.tile_surv;
+            I.stats.work_stair_candidates_total += o.stair;
+            I.stats.work_frontier_survivors_total += o.surv_total;
+            I.stats.work_frontier_peak_points = std::max(I.stats.work_frontier_peak_points, o.surv_peak);
+            I.stats.dominance_filtered_total += o.removed;
+            I.stats.layers_td += o.done;
+            I.stats.work_chained_layers += o.done;
+            arena_.release(s.pts);
+            arena_.release(s.off);
+            arena_.release(s.size);
+            const int b = o.done & 1;
+            arena_.release(r.buf[b ^ 1]);
+            s.off = reinterpret_cast<int64_t *>(r.buf[b]);
+            s.size = r.size(b);
+            s.sorted = r.sorted(b);
+            s.pts = r.pts(b);
+            s.layer += o.done;
+            s.slot_points = dev::kRunCap;
+        } else {
+            release_run(r);
+        }
+        if (s.layer == I.L - 1) {
+            arena_.release(arc_off);
+            s.counted = false;
+            I.result_n = o.final_size;
+            I.result.resize(static_cast<size_t>(o.final_size) * I.d * I.elem());
+            fetch(I, static_cast<const char *>(s.pts) + static_cast<size_t>(o.final_off) * I.d * I.elem());
+            I.stats.work_frontier_survivors_total += o.final_size;
+            I.stats.work_frontier_peak_points = std::max<int64_t>(I.stats.work_frontier_peak_points, o.final_size);
+            I.phase = Instance::DONE;
+        } else {
+            s.arc_off = arc_off;
+            s.big_list = big;
+            s.res = hres[r.count_idx];
+            s.counted = true;
+            s.score = s.res.total;
+            if (o.done > 0) {
+                I.stats.work_frontier_survivors_total += s.res.cur_total;
+                I.stats.work_frontier_peak_points = std::max(I.stats.work_frontier_peak_points, s.res.cur_total);
+            }
+        }
+    }
+    chained_layers_total_ += run_layers;
     for (size_t k = 0; k < ujobs.size(); ++k) {
         Instance &I = *ujob_inst[k];
         if (I.phase == Instance::DONE) continue;
@@ -2307,6 +2553,8 @@ int Engine::step() {
     if (trace_ && !chains.empty())
         std::fprintf(stderr, "[pmdd chain] requests=%zu layers=%d chained=%lld chain_ms=%.3f\n", chain_slots,
                      chain_layers_run, static_cast<long long>(chained_done), ms_chain);
+    if (trace_ && !runs.empty())
+        std::fprintf(stderr, "[pmdd run] requests=%zu layers=%lld\n", runs.size(), static_cast<long long>(run_layers));
     if (blocked && exps.empty() && ujobs.empty() && counts.empty()) {
         // nothing could move: the largest blocked request cannot fit next to the others
         fail(*blocked, PMDD_ERR_OOM, "device memory budget exhausted (layer does not fit)");

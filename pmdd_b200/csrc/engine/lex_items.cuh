@@ -107,11 +107,11 @@ __device__ __forceinline__ bool stair_covers(const T *s1, const T *s2, T q1, T q
     return at > 0 && s2[at - 1] >= q2;
 }
 
-// Filters destinations [i0, i1) of J; see above.  Every thread of a block of kLexThreads
-// calls it.
-template <typename T, bool RUN, class Last>
-__device__ __forceinline__ bool lex_items(LexSmem<T> &S, const ExpandJob &J, int32_t i0, int32_t i1, Last last) {
-    constexpr int NT = kLexThreads;
+// Filters destinations [i0, i1) of J; see above.  Every thread of a block of NT calls it;
+// `st` with RUN.
+template <typename T, int NT, bool RUN, class Last>
+__device__ __forceinline__ bool lex_items(LexSmem<T> &S, const ExpandJob &J, RunStage *st, int32_t i0, int32_t i1,
+                                          Last last) {
     TileItems &I = S.t;
     TileArcs &A = S.a;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -123,14 +123,14 @@ __device__ __forceinline__ bool lex_items(LexSmem<T> &S, const ExpandJob &J, int
     clk.start();
     bool called = false;
     for (int32_t ic = i0; ic < i1;) {
-        const int n_it = stage_items<NT, RUN>(I, J, ic, i1, true);
+        const int n_it = stage_items<NT, RUN>(I, J, st, ic, i1, true);
         if (n_it == 0) {
             if (tid == 0) atomicOr(J.err, kErrBounds);
             return false;
         }
         const int32_t total = I.tot_i;
         clk.lap(0);
-        stage_arcs<NT, RUN>(I, A, J, n_it);
+        stage_arcs<NT, RUN>(I, A, J, st, n_it);
         __syncthreads();
         clk.lap(1);
         assign_arcs<NT>(I, A);
@@ -138,7 +138,7 @@ __device__ __forceinline__ bool lex_items(LexSmem<T> &S, const ExpandJob &J, int
         // --- expand: candidate = parent point + arc weight (run order)
         for (int q = tid; q < total; q += NT) {
             const int x = A.tag[q];
-            const T *src = prev + (ld_live64<RUN>(J.prev_off + A.arc_nbr[x]) + (q - A.arc_pos[x])) * 3;
+            const T *src = prev + (parent_slot<RUN>(A, J, st, x) + (q - A.arc_pos[x])) * 3;
             const int32_t *w = J.weights + static_cast<int64_t>(A.arc_w[x]) * 3;
             S.p0[q] = ld_point<RUN>(src) + static_cast<T>(w[0]);
             S.p1[q] = ld_point<RUN>(src + 1) + static_cast<T>(w[1]);

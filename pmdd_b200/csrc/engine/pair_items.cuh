@@ -54,11 +54,11 @@ struct PairSmem {
     TileDraw draw;
 };
 
-// Filters destinations [i0, i1) of J; see above.  Every thread of a block of
-// pair_threads<D, T>() calls it.
-template <int D, typename T, bool RUN, class Last>
-__device__ __forceinline__ bool pair_items(PairSmem<D, T> &S, const ExpandJob &J, int32_t i0, int32_t i1, Last last) {
-    constexpr int NT = pair_threads<D, T>();
+// Filters destinations [i0, i1) of J; see above.  Every thread of a block of NT calls it;
+// `st` with RUN.
+template <int D, typename T, int NT, bool RUN, class Last>
+__device__ __forceinline__ bool pair_items(PairSmem<D, T> &S, const ExpandJob &J, RunStage *st, int32_t i0, int32_t i1,
+                                           Last last) {
     constexpr T kMost = sizeof(T) == 4 ? static_cast<T>(INT32_MAX) : static_cast<T>(INT64_MAX);
     TileItems &I = S.t;
     TileArcs &A = S.a;
@@ -67,19 +67,19 @@ __device__ __forceinline__ bool pair_items(PairSmem<D, T> &S, const ExpandJob &J
     T *outp = static_cast<T *>(J.out_pts);
     bool called = false;
     for (int32_t ic = i0; ic < i1;) {
-        const int n_it = stage_items<NT, RUN>(I, J, ic, i1, false);
+        const int n_it = stage_items<NT, RUN>(I, J, st, ic, i1, false);
         if (n_it == 0) {
             if (tid == 0) atomicOr(J.err, kErrBounds);
             return false;
         }
         const int32_t total = I.tot_i;
-        stage_arcs<NT, RUN>(I, A, J, n_it);
+        stage_arcs<NT, RUN>(I, A, J, st, n_it);
         __syncthreads();
         assign_arcs<NT>(I, A);
         // --- expand: candidate = parent point + arc weight
         for (int q = tid; q < total; q += NT) {
             const int x = A.tag[q];
-            const T *src = prev + (ld_live64<RUN>(J.prev_off + A.arc_nbr[x]) + (q - A.arc_pos[x])) * D;
+            const T *src = prev + (parent_slot<RUN>(A, J, st, x) + (q - A.arc_pos[x])) * D;
             const int32_t *w = J.weights + static_cast<int64_t>(A.arc_w[x]) * D;
             PackedPt<D, T> pt;
 #pragma unroll

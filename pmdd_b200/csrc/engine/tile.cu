@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(pair_threads<D, T>(), 1024 / pair_threads<D, T
     PairSmem<D, T> &S = *reinterpret_cast<PairSmem<D, T> *>(smem_raw);
     for_each_tile(S.draw, jobs, tile_bases, num_jobs, total_tiles, queue, tiles_dev,
                   [&](const ExpandJob &J, int32_t i0, int32_t i1, auto last) {
-                      return pair_items<D, T, false>(S, J, i0, i1, last);
+                      return pair_items<D, T, pair_threads<D, T>(), false>(S, J, nullptr, i0, i1, last);
                   });
 }
 

@@ -16,7 +16,7 @@ __global__ void __launch_bounds__(kLexThreads, sizeof(T) == 4 ? 4 : 2)
     LexSmem<T> &S = *reinterpret_cast<LexSmem<T> *>(smem_raw);
     for_each_tile(S.draw, jobs, tile_bases, num_jobs, total_tiles, queue, tiles_dev,
                   [&](const ExpandJob &J, int32_t i0, int32_t i1, auto last) {
-                      return lex_items<T, false>(S, J, i0, i1, last);
+                      return lex_items<T, kLexThreads, false>(S, J, nullptr, i0, i1, last);
                   });
 }
 

@@ -2,8 +2,8 @@
 // tile_lex.cu) and the layer-run kernel (run.cu): staging of destinations and arcs, the
 // arc of each candidate, survivor masks to slot positions.
 //
-// RUN: the frontiers and counts were written by other blocks of the same launch, so they
-// are read past the L1 cache.
+// RUN: the frontiers were written by other blocks of the same launch, so they are read past
+// the L1 cache; what the arcs lead to was gathered beforehand (RunStage).
 #pragma once
 
 #include <climits>
@@ -55,7 +55,7 @@ struct TileArcs {
     int16_t arc_pos[kTileArcCap + 1];    // staged arc -> first candidate position
     int16_t arc_item[kTileArcCap];       // staged arc -> staged destination
     int32_t arc_w[kTileArcCap];          // staged arc -> weight row
-    int32_t arc_nbr[kTileArcCap];        // staged arc -> job-local neighbour
+    int32_t arc_nbr[kTileArcCap];        // staged arc -> job-local neighbour (RUN: RunStage index)
 };
 
 // Phase clock (J.phase_clk, a diagnostic): thread 0 adds the cycles its block spent in
@@ -108,12 +108,26 @@ __device__ __forceinline__ int32_t block_exclusive_max(int32_t x, int32_t *warp_
     return r;
 }
 
+// A run's arcs of one layer and block (run.cu): candidate offsets, and per arc its weight row
+// and its neighbour's slot start and order flag.  J.arc_cand_off is `off`, J.arc_base the
+// first arc.
+constexpr int kRunRegion = 2048;         // arcs, and candidates, of a layer a block holds
+struct RunStage {
+    int64_t off[kRunRegion + 1];
+    int64_t src[kRunRegion];
+    int32_t nbr[kRunRegion];             // job-local neighbour
+    int32_t w[kRunRegion];
+    uint8_t sorted[kRunRegion];
+    int32_t over;                        // an oversized destination was staged
+};
+
 // Stages destinations [ic, i1) of J as far as their candidates and arcs fit and returns how
 // many (0: none, which well-formed plans rule out).  in_order: the pass writes frontiers
 // in lexicographic order.  Every thread calls it; S.tot_i / S.tot_a receive the candidates
 // and arcs.
 template <int NT, bool RUN>
-__device__ __forceinline__ int stage_items(TileItems &S, const ExpandJob &J, int32_t ic, int32_t i1, bool in_order) {
+__device__ __forceinline__ int stage_items(TileItems &S, const ExpandJob &J, RunStage *st, int32_t ic, int32_t i1,
+                                           bool in_order) {
     const int tid = threadIdx.x, lane = tid & 31;
     const int n_stage = min(kTileItemCap, i1 - ic);
     constexpr int PER = kTileItemCap / NT;
@@ -129,10 +143,11 @@ __device__ __forceinline__ int stage_items(TileItems &S, const ExpandJob &J, int
             const int32_t i = ic + k;
             const int32_t v = J.item_base + i;
             const int32_t a0 = J.item_arc_off[v], a1 = J.item_arc_off[v + 1];
-            const int64_t s = ld_live64<RUN>(J.arc_cand_off + (a0 - J.arc_base));
-            const int64_t c = ld_live64<RUN>(J.arc_cand_off + (a1 - J.arc_base)) - s;
+            const int64_t s = J.arc_cand_off[a0 - J.arc_base];
+            const int64_t c = J.arc_cand_off[a1 - J.arc_base] - s;
             J.out_off[i] = s;
             const bool resident = c > 0 && tile_resident(c, a1 - a0);
+            if (RUN && c > 0 && !resident) st->over = 1;
             if (c == 0) J.out_size[i] = 0;
             if (J.out_sorted) J.out_sorted[i] = (c == 0 || (resident && in_order)) ? 1 : 0;
             S.item_c0[k] = s;
@@ -196,7 +211,7 @@ __device__ __forceinline__ int stage_items(TileItems &S, const ExpandJob &J, int
 // Stages the arcs of the pass' n_it destinations and marks the ones with a run from an
 // unsorted parent; clears the tags.  A barrier must follow.
 template <int NT, bool RUN>
-__device__ __forceinline__ void stage_arcs(TileItems &S, TileArcs &A, const ExpandJob &J, int n_it) {
+__device__ __forceinline__ void stage_arcs(TileItems &S, TileArcs &A, const ExpandJob &J, const RunStage *st, int n_it) {
     const int tid = threadIdx.x;
     const int32_t total = S.tot_i, total_a = S.tot_a;
     for (int x = tid; x < total_a; x += NT) {
@@ -208,17 +223,29 @@ __device__ __forceinline__ void stage_arcs(TileItems &S, TileArcs &A, const Expa
         }
         const int k = lo;
         const int32_t a = S.item_a0g[k] + (x - S.item_arc0[k]);
-        const int64_t c0 = ld_live64<RUN>(J.arc_cand_off + (a - J.arc_base));
-        const int32_t nb = J.arc_nbr[a] - J.prev_base;
+        const int64_t c0 = J.arc_cand_off[a - J.arc_base];
         A.arc_pos[x] = static_cast<int16_t>(S.item_s[k] + (c0 - S.item_c0[k]));
-        A.arc_nbr[x] = nb;
-        A.arc_w[x] = J.arc_wrow[a];
         A.arc_item[x] = static_cast<int16_t>(k);
-        if (J.prev_sorted == nullptr || ld_live<RUN>(reinterpret_cast<const unsigned char *>(J.prev_sorted) + nb) == 0)
-            S.item_count[k] = 1;
+        if constexpr (RUN) {
+            A.arc_nbr[x] = a - J.arc_base;
+            A.arc_w[x] = st->w[a - J.arc_base];
+            if (st->sorted[a - J.arc_base] == 0) S.item_count[k] = 1;
+        } else {
+            const int32_t nb = J.arc_nbr[a] - J.prev_base;
+            A.arc_nbr[x] = nb;
+            A.arc_w[x] = J.arc_wrow[a];
+            if (J.prev_sorted == nullptr || J.prev_sorted[nb] == 0) S.item_count[k] = 1;
+        }
     }
     if (tid == 0) A.arc_pos[total_a] = static_cast<int16_t>(total);
     for (int q = tid; q < total; q += NT) A.tag[q] = -1;
+}
+
+// Slot start of staged arc x's neighbour.
+template <bool RUN>
+__device__ __forceinline__ int64_t parent_slot(const TileArcs &A, const ExpandJob &J, const RunStage *st, int x) {
+    if constexpr (RUN) return st->src[A.arc_nbr[x]];
+    else return J.prev_off[A.arc_nbr[x]];
 }
 
 // Each candidate's arc: every non-empty run's first position is marked, then a block-wide
