@@ -497,13 +497,19 @@ pmdd_resident *pmdd_resident_upload(const pmdd_dd *dds, int32_t count, int32_t d
     pack_all(*slot.engine, dds, R->tmpl);
     for (size_t i = 0; i < R->tmpl.size(); ++i) {
         pmdd::Instance &I = *R->tmpl[i];
-        if (!slot.engine->upload_dd(I)) {
+        if (!slot.engine->upload_dd(I, false)) {
             for (size_t k = 0; k <= i; ++k) slot.engine->release_dd(*R->tmpl[k]);
             write_err(err, errlen, slot.engine->ok() ? "DD set does not fit the device memory budget"
                                                      : slot.engine->error());
             return nullptr;
         }
         R->bytes += static_cast<int64_t>(I.dev_bytes);
+    }
+    if (!slot.engine->build_csrs(R->tmpl, 0)) {
+        for (auto &I : R->tmpl) slot.engine->release_dd(*I);
+        write_err(err, errlen, slot.engine->ok() ? "DD set does not fit the device memory budget"
+                                                 : slot.engine->error());
+        return nullptr;
     }
     if (cudaStreamSynchronize(slot.engine->stream()) != cudaSuccess) {
         write_err(err, errlen, "DD upload failed");
@@ -731,6 +737,7 @@ pmdd_resident *pmdd_resident_build_knapsack(const pmdd_knapsack *ks, int32_t cou
             cudaStreamSynchronize(st) != cudaSuccess)
             return give_up(std::string("knapsack build failed: ") + cudaGetErrorString(cudaGetLastError()));
         E.count_launches(1);
+        std::vector<int64_t> runs_ints(1, 0);  // flatten scratch of each instance
         for (int32_t k = 0; k < m; ++k) {
             const pmdd_knapsack &q = ks[i0 + k];
             const int32_t Lc = q.n + 1;
@@ -764,6 +771,7 @@ pmdd_resident *pmdd_resident_build_knapsack(const pmdd_knapsack *ks, int32_t cou
                                         q.n + 1);
             I->dd = static_cast<unsigned char *>(E.alloc(I->dev_bytes));
             if (!I->dd) return give_up("built DD set does not fit the device memory budget");
+            runs_ints.push_back(runs_ints.back() + pmdd::dev::kp_run_ints(layer_off.back()));
             pmdd::dev::KpBuildJob &J = jobs[k];
             J.layer_offsets = reinterpret_cast<int32_t *>(I->dd + I->off_layer);
             J.in_arc_offsets = reinterpret_cast<int32_t *>(I->dd + I->off_in);
@@ -776,12 +784,16 @@ pmdd_resident *pmdd_resident_build_knapsack(const pmdd_knapsack *ks, int32_t cou
             R->tmpl.push_back(std::move(I));
             R->widths.push_back({ow, on, rw, rn});
         }
+        int32_t *d_runs = static_cast<int32_t *>(dev_alloc(sizeof(int32_t) * static_cast<size_t>(runs_ints[m])));
+        if (!d_runs) return give_up("knapsack build scratch does not fit the device memory budget");
+        for (int32_t k = 0; k < m; ++k) jobs[k].runs = d_runs + runs_ints[k];
         if (cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(jobs[0]) * m, cudaMemcpyHostToDevice, st) != cudaSuccess ||
             pmdd::dev::launch_kp_flatten(d_jobs, m, max_layers, st) != cudaSuccess)
             return give_up(std::string("knapsack flatten failed: ") + cudaGetErrorString(cudaGetLastError()));
-        E.count_launches(1);
+        E.count_launches(2);
         for (int32_t k = 0; k < m; ++k)
-            if (!E.bind_dd(*R->tmpl[i0 + k])) return give_up(E.ok() ? "out-arc CSR failed" : E.error());
+            if (!E.bind_dd(*R->tmpl[i0 + k], false)) return give_up(E.ok() ? "out-arc CSR failed" : E.error());
+        if (!E.build_csrs(R->tmpl, static_cast<size_t>(i0))) return give_up(E.ok() ? "out-arc CSR failed" : E.error());
         if (cudaMemcpyAsync(hhdr.data(), d_hdr, sizeof(int32_t) * hhdr.size(), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
             return give_up(std::string("knapsack build failed: ") + cudaGetErrorString(cudaGetLastError()));
@@ -791,8 +803,9 @@ pmdd_resident *pmdd_resident_build_knapsack(const pmdd_knapsack *ks, int32_t cou
         E.release(d_scr);
         E.release(d_hdr);
         E.release(d_jobs);
+        E.release(d_runs);
         temps.erase(std::remove_if(temps.begin(), temps.end(),
-                                   [&](void *p) { return p == d_scr || p == d_hdr || p == d_jobs; }),
+                                   [&](void *p) { return p == d_scr || p == d_hdr || p == d_jobs || p == d_runs; }),
                     temps.end());
         i0 = i1;
     }

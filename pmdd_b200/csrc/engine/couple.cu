@@ -27,78 +27,83 @@ namespace pmdd {
 namespace dev {
 
 // ------------------------------------------------------------ out-arc CSR
-__global__ void out_degree_kernel(const int32_t *__restrict__ arc_src, int32_t num_arcs, int32_t *__restrict__ out_off) {
-    for (int32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < num_arcs; a += gridDim.x * blockDim.x)
-        atomicAdd(&out_off[arc_src[a] + 1], 1);
+// Of one DD (`one`, jobs nullptr) or of every DD of a set (grid.y), in four launches: zeroed
+// counts, out-degrees, their scan (a block per DD), scatter.
+__global__ void __launch_bounds__(256) csr_zero_kernel(const CsrJob *__restrict__ jobs, CsrJob one) {
+    const CsrJob &J = jobs ? jobs[blockIdx.y] : one;
+    for (int32_t v = blockIdx.x * 256 + threadIdx.x; v <= J.num_nodes; v += gridDim.x * 256) J.out_off[v] = 0;
 }
 
-// Inclusive scan of out_off[1..n] in place (one block; n is a node count).
-__global__ void __launch_bounds__(1024) csr_scan_kernel(int32_t *__restrict__ off, int32_t n, int32_t *__restrict__ cursor) {
+__global__ void __launch_bounds__(256) out_degree_kernel(const CsrJob *__restrict__ jobs, CsrJob one) {
+    const CsrJob &J = jobs ? jobs[blockIdx.y] : one;
+    for (int32_t a = blockIdx.x * 256 + threadIdx.x; a < J.num_arcs; a += gridDim.x * 256)
+        atomicAdd(&J.out_off[J.arc_src[a] + 1], 1);
+}
+
+// Inclusive scan of out_off[1..n] in place (one block per DD), 16 counts per thread at a
+// time: a single DD's scan is a serial chain of block scans, and 1024 counts per link took
+// 0.28 ms for 316 k nodes, 16384 take 0.03 ms.
+constexpr int kCsrPer = 16;
+__global__ void __launch_bounds__(1024) csr_scan_kernel(const CsrJob *__restrict__ jobs, CsrJob one) {
+    const CsrJob &J = jobs ? jobs[blockIdx.x] : one;
     __shared__ int32_t warp_buf[32];
-    __shared__ int32_t s_carry;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_carry = 0;
-    __syncthreads();
-    for (int32_t base = 0; base < n; base += 1024) {
-        const int32_t i = base + threadIdx.x;
-        int32_t x = i < n ? off[i + 1] : 0;
-        int32_t inc = x;
+    __shared__ int32_t total;
+    int32_t carry = 0;
+    for (int64_t base = 0; base < J.num_nodes; base += 1024 * kCsrPer) {
+        const int64_t i0 = base + static_cast<int64_t>(threadIdx.x) * kCsrPer;
+        int32_t x[kCsrPer], sum = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += y;
+        for (int r = 0; r < kCsrPer; ++r) {
+            x[r] = i0 + r < J.num_nodes ? J.out_off[i0 + r + 1] : 0;
+            sum += x[r];
         }
-        if (lane == 31) warp_buf[warp] = inc;
-        __syncthreads();
-        if (warp == 0) {
-            const int32_t w = warp_buf[lane];
-            int32_t winc = w;
+        int32_t run = carry + block_exclusive_scan<int32_t, 1024>(sum, warp_buf, &total);
+        carry += total;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int32_t y = __shfl_up_sync(0xffffffffu, winc, o);
-                if (lane >= o) winc += y;
+        for (int r = 0; r < kCsrPer; ++r) {
+            if (i0 + r < J.num_nodes) {
+                J.cursor[i0 + r] = run;  // start of the node's out-arcs
+                J.out_off[i0 + r + 1] = run + x[r];
             }
-            warp_buf[lane] = winc - w;
-        }
-        __syncthreads();
-        const int32_t val = s_carry + warp_buf[warp] + inc;
-        if (i < n) {
-            off[i + 1] = val;
-            cursor[i] = val - x;  // start of node i's out-arcs
-        }
-        __syncthreads();
-        if (threadIdx.x == 1023) s_carry = val;
-        __syncthreads();
-    }
-}
-
-__global__ void out_scatter_kernel(const int32_t *__restrict__ in_off, const int32_t *__restrict__ arc_src,
-                                   const int32_t *__restrict__ arc_w, int32_t num_nodes, int32_t *__restrict__ cursor,
-                                   int32_t *__restrict__ out_head, int32_t *__restrict__ out_w) {
-    for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < num_nodes; v += gridDim.x * blockDim.x) {
-        for (int32_t a = in_off[v]; a < in_off[v + 1]; ++a) {
-            const int32_t pos = atomicAdd(&cursor[arc_src[a]], 1);
-            out_head[pos] = v;
-            out_w[pos] = arc_w[a];
+            run += x[r];
         }
     }
 }
 
-cudaError_t launch_build_out_csr(const int32_t *in_off, const int32_t *arc_src, const int32_t *arc_w,
-                                 int32_t num_nodes, int32_t num_arcs, int32_t *out_off, int32_t *cursor,
-                                 int32_t *out_head, int32_t *out_w, cudaStream_t stream) {
-    cudaError_t e = cudaMemsetAsync(out_off, 0, sizeof(int32_t) * (static_cast<size_t>(num_nodes) + 1), stream);
-    if (e != cudaSuccess) return e;
-    if (num_arcs > 0) {
-        const int g = std::min(1184, (num_arcs + 255) / 256);
-        out_degree_kernel<<<g, 256, 0, stream>>>(arc_src, num_arcs, out_off);
+__global__ void __launch_bounds__(256) out_scatter_kernel(const CsrJob *__restrict__ jobs, CsrJob one) {
+    const CsrJob &J = jobs ? jobs[blockIdx.y] : one;
+    for (int32_t v = blockIdx.x * 256 + threadIdx.x; v < J.num_nodes; v += gridDim.x * 256) {
+        for (int32_t a = J.in_off[v]; a < J.in_off[v + 1]; ++a) {
+            const int32_t pos = atomicAdd(&J.cursor[J.arc_src[a]], 1);
+            J.out_head[pos] = v;
+            J.out_w[pos] = J.arc_w[a];
+        }
     }
-    csr_scan_kernel<<<1, 1024, 0, stream>>>(out_off, num_nodes, cursor);
-    if (num_nodes > 0) {
-        const int g = std::min(1184, (num_nodes + 255) / 256);
-        out_scatter_kernel<<<g, 256, 0, stream>>>(in_off, arc_src, arc_w, num_nodes, cursor, out_head, out_w);
-    }
+}
+
+static cudaError_t launch_csr(const CsrJob *jobs, const CsrJob &one, int count, int32_t max_nodes, int32_t max_arcs,
+                              cudaStream_t stream) {
+    if (count <= 0) return cudaSuccess;
+    const int cap = std::max(1, 1184 / std::min(count, 64));
+    const dim3 gn(std::min(cap, max_nodes / 256 + 1), count), ga(std::min(cap, max_arcs / 256 + 1), count);
+    csr_zero_kernel<<<gn, 256, 0, stream>>>(jobs, one);
+    out_degree_kernel<<<ga, 256, 0, stream>>>(jobs, one);
+    csr_scan_kernel<<<count, 1024, 0, stream>>>(jobs, one);
+    out_scatter_kernel<<<gn, 256, 0, stream>>>(jobs, one);
     return cudaGetLastError();
+}
+
+cudaError_t launch_build_out_csr(const CsrJob &job, cudaStream_t stream) {
+    return launch_csr(nullptr, job, 1, job.num_nodes, job.num_arcs, stream);
+}
+
+cudaError_t launch_build_out_csrs(const CsrJob *jobs, int count, int32_t max_nodes, int32_t max_arcs,
+                                  cudaStream_t stream) {
+    for (int at = 0; at < count; at += 32768) {  // grid.y
+        const cudaError_t e = launch_csr(jobs + at, CsrJob{}, std::min(count - at, 32768), max_nodes, max_arcs, stream);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 // ------------------------------------------------------------------ coupling

@@ -49,9 +49,22 @@ inline size_t couple_bytes(int64_t ucap, int d, size_t elem) {
     return 4 * pts + 2 * idx;
 }
 
-cudaError_t launch_build_out_csr(const int32_t *in_off, const int32_t *arc_src, const int32_t *arc_w,
-                                 int32_t num_nodes, int32_t num_arcs, int32_t *out_off, int32_t *cursor,
-                                 int32_t *out_head, int32_t *out_w, cudaStream_t stream);
+// The bottom-up (outgoing-arc) CSR of a DD: arc order within a node unspecified.
+struct CsrJob {
+    const int32_t *in_off;
+    const int32_t *arc_src;
+    const int32_t *arc_w;
+    int32_t num_nodes, num_arcs;
+    int32_t *out_off;   // [num_nodes + 1]
+    int32_t *cursor;    // [num_nodes] scratch
+    int32_t *out_head;  // [num_arcs]
+    int32_t *out_w;     // [num_arcs]
+};
+constexpr int kCsrLaunches = 4;
+cudaError_t launch_build_out_csr(const CsrJob &job, cudaStream_t stream);
+// Of many DDs at once (device array).
+cudaError_t launch_build_out_csrs(const CsrJob *jobs, int count, int32_t max_nodes, int32_t max_arcs,
+                                  cudaStream_t stream);
 
 // One coupling round for `num_jobs` jobs of one (d, wide) group.  A seed round counts the
 // units and products, orders the cutset's frontiers, and appends, per cutset node, the sums

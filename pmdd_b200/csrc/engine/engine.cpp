@@ -465,13 +465,14 @@ const TspStructure *Engine::tsp_structure(int n, std::string *err) {
     S->out_head = at(o_oh);
     S->out_w = at(o_ow);
     S->cursor = at(o_cur);
-    ok = ok && cuda_ok(dev::launch_build_out_csr(S->in_off, S->arc_src, S->arc_w, S->N, S->A, S->out_off, S->cursor,
-                                                 S->out_head, S->out_w, stream_),
+    ok = ok && cuda_ok(dev::launch_build_out_csr({S->in_off, S->arc_src, S->arc_w, S->N, S->A, S->out_off, S->cursor,
+                                                  S->out_head, S->out_w},
+                                                 stream_),
                        "TSP out-arc CSR");
     ok = ok && cuda_ok(cudaMemcpyAsync(&h_err, d_err, sizeof(int32_t), cudaMemcpyDeviceToHost, stream_), "TSP check") &&
          cuda_ok(cudaStreamSynchronize(stream_), "TSP structure");
-    launches_ += nl + 3;
-    g_total_launches += nl + 3;
+    launches_ += nl + dev::kCsrLaunches;
+    g_total_launches += nl + dev::kCsrLaunches;
     arena_.release(scratch);
     if (!ok || h_err != 0) {
         arena_.release(S->mem);
@@ -855,16 +856,45 @@ bool Engine::make_current() {
     return cuda_ok(cudaSetDevice(device_), "cudaSetDevice");
 }
 
-bool Engine::upload_dd(Instance &I) {
+bool Engine::upload_dd(Instance &I, bool build_csr) {
     if (!make_current()) return false;
     I.dd = static_cast<unsigned char *>(arena_.alloc(I.dev_bytes));
     if (!I.dd) return false;
     if (!cuda_ok(cudaMemcpyAsync(I.dd, I.blob_src ? I.blob_src : I.blob.data(), I.blob_bytes, cudaMemcpyHostToDevice, stream_), "DD upload"))
         return false;
-    return bind_dd(I);
+    return bind_dd(I, build_csr);
 }
 
-bool Engine::bind_dd(Instance &I) {
+static dev::CsrJob csr_job(const Instance &I) {
+    return {I.d_in_off, I.d_arc_src, I.d_arc_w, I.N, I.A, I.d_out_off, I.d_cursor, I.d_out_head, I.d_out_w};
+}
+
+bool Engine::build_csrs(const std::vector<std::unique_ptr<Instance>> &insts, size_t from) {
+    std::vector<dev::CsrJob> jobs;
+    int32_t max_nodes = 0, max_arcs = 0;
+    for (size_t i = from; i < insts.size(); ++i) {
+        const Instance &I = *insts[i];
+        if (I.tsp || !I.with_out_csr) continue;
+        jobs.push_back(csr_job(I));
+        max_nodes = std::max(max_nodes, I.N);
+        max_arcs = std::max(max_arcs, I.A);
+    }
+    if (jobs.empty()) return true;
+    void *d = arena_.alloc(sizeof(dev::CsrJob) * jobs.size());
+    if (!d) return false;
+    // (the copy from pageable memory has left `jobs` when it returns)
+    const bool ok = cuda_ok(cudaMemcpyAsync(d, jobs.data(), sizeof(dev::CsrJob) * jobs.size(), cudaMemcpyHostToDevice,
+                                            stream_),
+                            "out-arc CSR") &&
+                    cuda_ok(dev::launch_build_out_csrs(static_cast<const dev::CsrJob *>(d),
+                                                       static_cast<int>(jobs.size()), max_nodes, max_arcs, stream_),
+                            "out-arc CSR");
+    arena_.release(d);
+    count_launches(dev::kCsrLaunches);
+    return ok;
+}
+
+bool Engine::bind_dd(Instance &I, bool build_csr) {
     if (I.tsp) {  // shared structure: only the weight table is the instance's own
         const TspStructure &S = *I.tsp;
         I.d_layer_off = reinterpret_cast<const int32_t *>(S.mem);  // the structure's first array
@@ -898,12 +928,9 @@ bool Engine::bind_dd(Instance &I) {
         I.d_out_w = reinterpret_cast<int32_t *>(I.dd + off);
         off = align256(off + sizeof(int32_t) * static_cast<size_t>(I.A));
         I.d_cursor = reinterpret_cast<int32_t *>(I.dd + off);
-        if (!cuda_ok(dev::launch_build_out_csr(I.d_in_off, I.d_arc_src, I.d_arc_w, I.N, I.A, I.d_out_off, I.d_cursor,
-                                               I.d_out_head, I.d_out_w, stream_),
-                     "out-arc CSR"))
-            return false;
-        launches_ += 3;
-        g_total_launches += 3;
+        if (!build_csr) return true;
+        if (!cuda_ok(dev::launch_build_out_csr(csr_job(I), stream_), "out-arc CSR")) return false;
+        count_launches(dev::kCsrLaunches);
     }
     return true;
 }

@@ -279,13 +279,15 @@ class Engine {
     KernelTimes kernel_times() const { return ktimes_; }
     // Device copy of a prepared request's DD (with the bottom-up CSR) that stays in
     // the arena until release_dd(); requests then share it via external_dd.
-    bool upload_dd(Instance &I);
+    bool upload_dd(Instance &I, bool build_csr = true);
     // Makes this engine's device current on the calling thread (a thread may drive the
     // engines of several devices); every entry below that launches work calls it.
     bool make_current();
     // Device pointers of a DD whose arrays are in I.dd (uploaded or built on the device),
-    // and its bottom-up CSR when the instance carries one.
-    bool bind_dd(Instance &I);
+    // and its bottom-up CSR when the instance carries one (not with build_csr false: build_csrs
+    // then makes those of insts[from..] together).
+    bool bind_dd(Instance &I, bool build_csr = true);
+    bool build_csrs(const std::vector<std::unique_ptr<Instance>> &insts, size_t from);
     // The structure of n-city TSP MDDs on this engine's device, built on first use and
     // kept for the engine's life; nullptr (with *err) if it cannot be built.
     const TspStructure *tsp_structure(int n, std::string *err);

@@ -1,4 +1,5 @@
 // Exact knapsack BDDs built on the device: see kpbuild.cuh for the construction.
+#include <algorithm>
 #include <climits>
 
 #include "kpbuild.cuh"
@@ -165,102 +166,174 @@ __global__ void __launch_bounds__(NT) kp_reduce_kernel(const KpBuildJob *jobs) {
     }
 }
 
+// Block (l, k): the arcs of instance k from layer l into layer l + 1; block (0, k) also the
+// layer offsets, the weight table and the root.  Layers do not depend on one another, and
+// a run of more than kLongRun parents is sorted by the whole block: one thread's insertion
+// of a layer's longest run (hundreds of parents, its square in dependent global accesses)
+// took 20 of the 37 ms that 64 instances of 20..60 items spent in construction kernels.
+constexpr int kLongRun = 12;
+constexpr int kLongStage = 2048;
+
 __global__ void __launch_bounds__(NT) kp_flatten_kernel(const KpBuildJob *jobs) {
-    extern __shared__ int32_t lo[];  // [n+2] layer offsets
-    const KpBuildJob &J = jobs[blockIdx.x];
+    const KpBuildJob &J = jobs[blockIdx.y];
     __shared__ int32_t warp_buf[32];
-    __shared__ int32_t total;
-    const int n = J.n, d = J.nobjs, tid = threadIdx.x;
+    __shared__ int32_t total, s_long, s_arc_base, s_lo, s_nodes;
+    __shared__ int32_t stage[kLongStage];
+    const int n = J.n, d = J.nobjs, tid = threadIdx.x, l = blockIdx.x;
+    if (l >= n) return;
     const int64_t S = static_cast<int64_t>(J.cap) + 1;
-    if (tid == 0) {
-        int32_t acc = 0;
-        for (int l = 0; l <= n; ++l) {
-            lo[l] = acc;
-            acc += J.classes[l];
+    if (tid < 32) {  // nodes before layer l, in all, and arcs into the layers up to l
+        int32_t lo = 0, nodes = 0, arcs = 0;
+        for (int q = tid; q <= n; q += 32) {
+            const int32_t k = J.classes[q];
+            nodes += k;
+            if (q < l) lo += k;
+            if (q <= l) arcs += J.arcs_into[q];
         }
-        lo[n + 1] = acc;
+        for (int o = 16; o > 0; o >>= 1) {
+            lo += __shfl_xor_sync(0xffffffffu, lo, o);
+            nodes += __shfl_xor_sync(0xffffffffu, nodes, o);
+            arcs += __shfl_xor_sync(0xffffffffu, arcs, o);
+        }
+        if (tid == 0) {
+            s_lo = lo;
+            s_nodes = nodes;
+            s_arc_base = arcs;
+            s_long = 0;
+        }
     }
     __syncthreads();
-    for (int l = tid; l <= n + 1; l += NT) J.layer_offsets[l] = lo[l];
-    for (int r = tid; r <= n; r += NT)
-        for (int o = 0; o < d; ++o) J.weights[r * d + o] = r == 0 ? 0 : J.profit[o * n + (r - 1)];
-    if (tid == 0) {
-        J.in_arc_offsets[0] = 0;
-        J.in_arc_offsets[1] = 0;  // the root has no incoming arcs
-        J.min_weight[0] = 0;
+    const int32_t lo = s_lo, N = s_nodes;
+    if (tid == 0) J.layer_offsets[l] = lo;
+    if (l == 0) {
+        for (int r = tid; r <= n; r += NT)
+            for (int o = 0; o < d; ++o) J.weights[r * d + o] = r == 0 ? 0 : J.profit[o * n + (r - 1)];
+        if (tid == 0) {
+            J.layer_offsets[n] = N - 1;  // the terminal
+            J.layer_offsets[n + 1] = N;
+            J.in_arc_offsets[0] = 0;
+            J.in_arc_offsets[1] = 0;  // the root has no incoming arcs
+            J.sd_order[N - 1] = 0;
+        }
     }
-    int32_t *s1 = J.tmp, *e1 = J.tmp + S, *s0 = J.tmp + 2 * S, *e0 = J.tmp + 3 * S, *deg = J.tmp + 4 * S;
-    int32_t arc_base = 0;
+    const int32_t Kp = J.classes[l], Kc = J.classes[l + 1];
+    const int32_t base = lo + Kp;
+    int32_t *s1 = J.runs + base, *e1 = s1 + N, *s0 = e1 + N, *e0 = s0 + N, *deg = e0 + N;
+    int32_t *longs = J.idx + l * S;  // children with a long run (the states are done with)
+    const int32_t *cnew = J.cls_new + l * S, *c0 = J.cls_c0 + l * S, *c1 = J.cls_c1 + l * S;
+    for (int32_t v = tid; v < Kc; v += NT) {
+        s1[v] = -1;
+        e1[v] = -1;
+        s0[v] = -1;
+        e0[v] = -1;
+    }
     __syncthreads();
-    for (int l = 0; l < n; ++l) {
-        const int32_t Kp = J.classes[l], Kc = J.classes[l + 1];
-        const int32_t *cnew = J.cls_new + l * S, *c0 = J.cls_c0 + l * S, *c1 = J.cls_c1 + l * S;
-        const int32_t wl = J.w[l];
-        for (int32_t v = tid; v < Kc; v += NT) {
-            s1[v] = -1;
-            e1[v] = -1;
-            s0[v] = -1;
-            e0[v] = -1;
+    // the parents of a child through one arc type are a run of classes in state order
+    for (int32_t p = tid; p < Kp; p += NT) {
+        const int32_t v1 = c1[p], v0 = c0[p];
+        if (v1 >= 0 && v1 < Kc) {
+            if (p == 0 || c1[p - 1] != v1) s1[v1] = p;
+            if (p == Kp - 1 || c1[p + 1] != v1) e1[v1] = p;
         }
-        __syncthreads();
-        // the parents of a child through one arc type are a run of classes in state order
-        for (int32_t p = tid; p < Kp; p += NT) {
-            const int32_t v1 = c1[p], v0 = c0[p];
-            if (v1 >= 0 && v1 < Kc) {
-                if (p == 0 || c1[p - 1] != v1) s1[v1] = p;
-                if (p == Kp - 1 || c1[p + 1] != v1) e1[v1] = p;
-            }
-            if (v0 >= 0 && v0 < Kc) {
-                if (p == 0 || c0[p - 1] != v0) s0[v0] = p;
-                if (p == Kp - 1 || c0[p + 1] != v0) e0[v0] = p;
-            }
+        if (v0 >= 0 && v0 < Kc) {
+            if (p == 0 || c0[p - 1] != v0) s0[v0] = p;
+            if (p == Kp - 1 || c0[p + 1] != v0) e0[v0] = p;
         }
-        __syncthreads();
-        for (int32_t v = tid; v < Kc; v += NT)
-            deg[v] = (s1[v] >= 0 ? e1[v] - s1[v] + 1 : 0) + (s0[v] >= 0 ? e0[v] - s0[v] + 1 : 0);
-        __syncthreads();
-        const int32_t layer_arcs = block_scan_array(deg, Kc, warp_buf, &total);
-        for (int32_t v = tid; v < Kc; v += NT) {
-            int32_t a = arc_base + deg[v];
-            int32_t mw = INT_MAX;
+        J.sd_order[lo + (Kp - 1 - p)] = cnew[p];
+    }
+    __syncthreads();
+    for (int32_t v = tid; v < Kc; v += NT)
+        deg[v] = (s1[v] >= 0 ? e1[v] - s1[v] + 1 : 0) + (s0[v] >= 0 ? e0[v] - s0[v] + 1 : 0);
+    __syncthreads();
+    block_scan_array(deg, Kc, warp_buf, &total);
+    for (int32_t v = tid; v < Kc; v += NT) {
+        int32_t a = s_arc_base + deg[v];
+        bool any_long = false;
 #pragma unroll 1
-            for (int t = 1; t >= 0; --t) {
-                const int32_t sb = t ? s1[v] : s0[v], se = t ? e1[v] : e0[v];
-                if (sb < 0) continue;
-                const int32_t a0 = a;
-                for (int32_t p = sb; p <= se; ++p) {
-                    const int32_t u = cnew[p];
-                    // insertion into [a0, a) kept ascending by parent id
-                    int32_t q = a;
-                    while (q > a0 && J.arc_src[q - 1] > lo[l] + u) {
-                        J.arc_src[q] = J.arc_src[q - 1];
-                        --q;
+        for (int t = 1; t >= 0; --t) {
+            const int32_t sb = t ? s1[v] : s0[v], se = t ? e1[v] : e0[v];
+            if (sb < 0) continue;
+            const int32_t a0 = a;
+            if (se - sb >= kLongRun) {  // for the whole block
+                any_long = true;
+                a += se - sb + 1;
+                continue;
+            }
+            for (int32_t p = sb; p <= se; ++p) {
+                const int32_t u = cnew[p];
+                // insertion into [a0, a) kept ascending by parent id
+                int32_t q = a;
+                while (q > a0 && J.arc_src[q - 1] > lo + u) {
+                    J.arc_src[q] = J.arc_src[q - 1];
+                    --q;
+                }
+                J.arc_src[q] = lo + u;
+                J.arc_weight[a] = t ? 1 + l : 0;
+                ++a;
+            }
+        }
+        J.in_arc_offsets[base + v + 1] = a;
+        if (any_long) longs[atomicAdd(&s_long, 1)] = v;
+    }
+    __syncthreads();
+    // long runs: each parent's place is the number of smaller ids in the run
+    const int32_t num_long = s_long;
+    for (int32_t i = 0; i < num_long; ++i) {
+        const int32_t v = longs[i];
+        int32_t a = s_arc_base + deg[v];
+#pragma unroll 1
+        for (int t = 1; t >= 0; --t) {
+            const int32_t sb = t ? s1[v] : s0[v], se = t ? e1[v] : e0[v];
+            if (sb < 0) continue;
+            const int32_t len = se - sb + 1;
+            if (len > kLongRun) {
+                for (int32_t p0 = 0; p0 < len; p0 += NT) {
+                    const int32_t p = p0 + tid;
+                    const int32_t u = p < len ? cnew[sb + p] : 0;
+                    int32_t place = 0;
+                    for (int32_t q0 = 0; q0 < len; q0 += kLongStage) {
+                        const int32_t m = min(kLongStage, len - q0);
+                        __syncthreads();
+                        for (int32_t q = tid; q < m; q += NT) stage[q] = cnew[sb + q0 + q];
+                        __syncthreads();
+                        if (p < len)
+                            for (int32_t q = 0; q < m; ++q) place += stage[q] < u ? 1 : 0;
                     }
-                    J.arc_src[q] = lo[l] + u;
-                    J.arc_weight[a] = t ? 1 + l : 0;
-                    mw = min(mw, J.min_weight[lo[l] + u] + (t ? wl : 0));
-                    ++a;
+                    if (p < len) {
+                        J.arc_src[a + place] = lo + u;
+                        J.arc_weight[a + place] = t ? 1 + l : 0;
+                    }
                 }
             }
-            J.in_arc_offsets[lo[l + 1] + v + 1] = a;
-            J.min_weight[lo[l + 1] + v] = mw == INT_MAX ? 0 : mw;
+            a += len;
         }
-        arc_base += layer_arcs;
+    }
+}
+
+__global__ void __launch_bounds__(NT) kp_minw_kernel(const KpBuildJob *jobs) {
+    const KpBuildJob &J = jobs[blockIdx.x];
+    const int n = J.n, tid = threadIdx.x;
+    const int64_t S = static_cast<int64_t>(J.cap) + 1;
+    const int32_t *lo = J.layer_offsets;
+    if (tid == 0) J.min_weight[0] = 0;
+    __syncthreads();
+    for (int l = 0; l < n; ++l) {
+        const int32_t wl = J.w[l];
+        for (int32_t v = lo[l + 1] + tid; v < lo[l + 2]; v += NT) {
+            int32_t mw = INT_MAX;
+            for (int32_t a = J.in_arc_offsets[v]; a < J.in_arc_offsets[v + 1]; ++a)
+                mw = min(mw, J.min_weight[J.arc_src[a]] + (J.arc_weight[a] != 0 ? wl : 0));
+            J.min_weight[v] = mw == INT_MAX ? 0 : mw;
+        }
         __syncthreads();
     }
     // min_weight order per layer (descending, ties by id): the reverse state order of the
     // classes, since a class's min_weight is its smallest reachable state
-    for (int l = 0; l <= n; ++l) {
+    for (int l = 0; l < n; ++l) {
         const int32_t K = J.classes[l];
-        if (l == n) {
-            if (tid == 0) J.sd_order[lo[n]] = 0;
-            break;
-        }
         const int32_t *cnew = J.cls_new + l * S;
-        for (int32_t p = tid; p < K; p += NT) {
-            J.sd_order[lo[l] + (K - 1 - p)] = cnew[p];
-            if (p + 1 < K && J.min_weight[lo[l] + cnew[p]] >= J.min_weight[lo[l] + cnew[p + 1]]) atomicMax(J.err, 2);
-        }
+        for (int32_t p = tid; p + 1 < K; p += NT)
+            if (J.min_weight[lo[l] + cnew[p]] >= J.min_weight[lo[l] + cnew[p + 1]]) atomicMax(J.err, 2);
     }
 }
 
@@ -272,13 +345,9 @@ cudaError_t launch_kp_reduce(const KpBuildJob *jobs, int count, cudaStream_t str
 
 cudaError_t launch_kp_flatten(const KpBuildJob *jobs, int count, int max_layers, cudaStream_t stream) {
     if (count <= 0) return cudaSuccess;
-    const size_t smem = sizeof(int32_t) * (static_cast<size_t>(max_layers) + 2);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kp_flatten_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-    }
-    kp_flatten_kernel<<<count, NT, smem, stream>>>(jobs);
+    for (int at = 0; at < count; at += 32768)  // grid.y
+        kp_flatten_kernel<<<dim3(max_layers, std::min(count - at, 32768)), NT, 0, stream>>>(jobs + at);
+    kp_minw_kernel<<<count, NT, 0, stream>>>(jobs);
     return cudaGetLastError();
 }
 

@@ -14,12 +14,13 @@
 //                     agree merge.  Completion sets shrink as s grows, so the merged states
 //                     form runs of consecutive reachable states; a class is numbered by the
 //                     smallest old index among its states (first occurrence).
-//  kp_flatten_kernel  top-down again over the classes: in-arc CSR (1-arcs, then 0-arcs,
-//                     each by parent id; the parents of one child through one arc type are
-//                     a run of consecutive classes in state order), min_weight (min over
-//                     in-arcs), the weight table, and the min_weight order per layer
-//                     (descending; min_weight is the smallest state of a class, so it is
-//                     the reverse state order -- checked).
+//  kp_flatten_kernel  a block per layer and instance: in-arc CSR (1-arcs, then 0-arcs, each by
+//                     parent id; the parents of one child through one arc type are a run of
+//                     consecutive classes in state order), the weight table, and the
+//                     min_weight order per layer (descending; min_weight is the smallest
+//                     state of a class, so it is the reverse state order).
+//  kp_minw_kernel     a block per instance, layer by layer: min_weight (min over in-arcs), and
+//                     the check of that order.
 #pragma once
 
 #include "common.cuh"
@@ -47,6 +48,7 @@ struct KpBuildJob {
     int32_t *classes;        // [n+1] reduced layer sizes
     int32_t *arcs_into;      // [n+1] arcs into each layer
     int32_t *err;            // 0 ok; 1 inconsistent counts; 2 min_weight order check failed
+    int32_t *runs;           // kp_flatten_kernel scratch: kp_run_ints(nodes)
     // the flat DD (kp_flatten_kernel), pmdd_dd layout
     int32_t *layer_offsets, *in_arc_offsets, *arc_src, *arc_weight, *weights, *min_weight, *sd_order;
 };
@@ -56,6 +58,10 @@ inline int64_t kp_scratch_ints(int32_t n, int32_t cap) {
     const int64_t S = static_cast<int64_t>(cap) + 1;
     return (4 * (static_cast<int64_t>(n) + 1) + 10) * S;
 }
+
+// Flatten scratch of a DD of N nodes: per node the first and last parent class of either arc
+// type, and its in-degree.
+inline int64_t kp_run_ints(int32_t N) { return 5 * static_cast<int64_t>(N); }
 
 cudaError_t launch_kp_reduce(const KpBuildJob *jobs, int count, cudaStream_t stream);
 cudaError_t launch_kp_flatten(const KpBuildJob *jobs, int count, int max_layers, cudaStream_t stream);
