@@ -139,9 +139,8 @@ typedef struct pmdd_stats {
     int64_t work_tile_candidates_total;  /* candidates filtered in shared-memory tiles */
     int64_t work_tile_survivors_total;   /* survivors the tile kernel wrote */
     int64_t tile_launches;               /* expand+filter tile kernels this call launched */
-    int64_t work_stair_candidates_total; /* three objectives: candidates of destinations filtered by a
-                                            staircase warp (tiles above the pairwise limit, and
-                                            oversized destinations with sorted runs) */
+    int64_t work_stair_candidates_total; /* three objectives: candidates of tile destinations above the
+                                            pairwise limit, filtered by staircases */
     int64_t work_chained_layers;         /* layers expanded by chained steps (several layers between two
                                             host read-backs, for steps with few candidates) */
 } pmdd_stats;

@@ -21,7 +21,10 @@
 // The pass replaced one that tested every candidate against 4*sqrt(n) pivots and then
 // compared all pairs of the rest (one B200, oversized path per enumeration, before -> now):
 // TSP d=5 n=13 38.7 -> 9.6 ms (23.7 M candidates), KP d=4 n=60 18.8 -> 6.0 ms (17.7 M),
-// KP d=7 n=25 1.14 -> 0.56 ms.
+// KP d=7 n=25 1.14 -> 0.56 ms.  It also took over the three-objective destinations with
+// sorted runs, which one staircase warp each walked in lexicographic order: oversized
+// path of the 192-instance stream 21.3 -> 11.9 ms, against 2 ms more in the tiles, whose
+// runs from these parents arrive unsorted.
 #include "big_common.cuh"
 #include "kernels.cuh"
 #include "maxima.cuh"
@@ -240,12 +243,7 @@ static cudaError_t launch_big_t(const BigLaunch &L, cudaStream_t stream) {
         const cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(big_sfs_kernel<D, T>), Cfg::kSmem);
         if (e != cudaSuccess) return e;
     }
-    const bool lex = D == 3 && L.lex_big;
-    if (lex) {
-        cudaError_t e = launch_big_lex_rank(sizeof(T) == 8, L, stream);
-        for (int r = 0; e == cudaSuccess && r < L.lex_rounds; ++r) e = launch_big_lex_merge(sizeof(T) == 8, L, r, stream);
-        if (e != cudaSuccess) return e;
-    } else {
+    {
         const int64_t want = (L.total + kFlatThreads - 1) / kFlatThreads;
         const unsigned grid = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(want, int64_t(L.sms) * 32)));
         big_expand_kernel<D, T><<<grid, kFlatThreads, 0, stream>>>(L.jobs, L.job_bases, L.num_jobs, L.total, L.pass);
@@ -266,7 +264,6 @@ static cudaError_t launch_big_t(const BigLaunch &L, cudaStream_t stream) {
         const cudaError_t e = launch_maxima<D, T>(BigSrc<T>{L.jobs, plan, L.mark_cap}, L.mark_cap, chunks, stream);
         if (e != cudaSuccess) return e;
     }
-    if (lex) return launch_big_lex_filter(sizeof(T) == 8, L, stream);
     return cudaGetLastError();
 }
 

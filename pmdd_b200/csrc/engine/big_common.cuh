@@ -1,4 +1,4 @@
-// Shared device helpers of the oversized-destination paths (big.cu, big_lex.cu): the
+// Shared device helpers of the oversized-destination paths (big.cu): the
 // destination behind a work item or a flat candidate index of one scratch pass, and the
 // arc run a candidate belongs to.
 #pragma once
@@ -34,15 +34,6 @@ __device__ __forceinline__ unsigned char *big_slab(const ExpandJob &J, int64_t s
     return static_cast<unsigned char *>(J.big_slab) + soff * static_cast<int64_t>(2 * D * sizeof(T));
 }
 
-// Destinations of three objectives whose runs all come from sorted frontiers, at most
-// J.lex_max_arcs of them: the lexicographic path (big_lex.cu) filters these.
-__device__ __forceinline__ bool lex_eligible(const ExpandJob &J, const BigItem &B) {
-    if (J.prev_sorted == nullptr || B.a1 - B.a0 > J.lex_max_arcs) return false;
-    for (int32_t a = B.a0; a < B.a1; ++a)
-        if (J.prev_sorted[J.arc_nbr[a] - J.prev_base] == 0) return false;
-    return true;
-}
-
 // The destination of work item W, if pass `pass` takes it (its scratch offset lies in the
 // pass's window); its scratch offset is then re-based to the window.
 __device__ __forceinline__ bool big_item(const ExpandJob &J, const BigWork &W, int64_t pass, BigItem *b) {
@@ -50,7 +41,7 @@ __device__ __forceinline__ bool big_item(const ExpandJob &J, const BigWork &W, i
     const int64_t s = J.big_list[2 * W.big + 1];
     if (s < lo || s >= lo + J.big_window) return false;
     fill_item(J, W.big, lo, b);
-    return !(J.lex_big && lex_eligible(J, *b));
+    return true;
 }
 
 __device__ __forceinline__ int find_job(const int64_t *bases, int n, int64_t g) {

@@ -48,19 +48,6 @@ __host__ __device__ constexpr bool tile_resident(int64_t candidates, int64_t arc
     return candidates <= kSmallMax && arcs <= kTileArcCap / 2;
 }
 
-// Oversized three-objective destinations in lexicographic order (big_lex.cu): up to
-// kBigDirectArcs runs each candidate is ranked against the other runs directly; beyond,
-// ceil(log2(runs)) merge rounds of neighbouring run groups sort the destination; more
-// than ExpandJob::lex_max_arcs (at most kBigLexMaxArcs) runs take the pivot/mark path.
-constexpr int kBigDirectArcs = 16;
-constexpr int kBigLexMaxArcs = 4096;
-__host__ __device__ inline int lex_merge_rounds(int arcs) {
-    int r = 0;
-    if (arcs > kBigDirectArcs)
-        while ((1 << r) < arcs) ++r;
-    return r;
-}
-
 constexpr int kCountThreads = 1024;
 constexpr int kBigThreads = 256;
 constexpr int kBigJTile = 1024;       // candidates per shared-memory comparison tile
@@ -115,9 +102,6 @@ struct ExpandJob {
     uint8_t *out_sorted;
     int32_t pair_max;              // lexicographic tiles: destinations of at most this many
                                    // candidates are checked pairwise, larger ones by a staircase warp
-    int32_t lex_big;               // 1: oversized destinations with sorted runs take big_lex.cu
-    int32_t lex_max_arcs;          // oversized destinations of at most this many runs (and at
-                                   // most kBigLexMaxArcs) take big_lex.cu
     unsigned long long *phase_clk; // diagnostic: cycles per tile phase (lexicographic tiles), or nullptr
 };
 

@@ -606,8 +606,6 @@ Engine::Engine(int device, int64_t budget_bytes, int max_slots, int stream_prior
     if (cr && *cr) chain_max_requests_ = std::max<int64_t>(0, std::atoll(cr));
     const char *cm = std::getenv("PMDD_CHAIN_MAX_CAND");
     if (cm && *cm) chain_max_cand_ = std::max<int64_t>(0, std::atoll(cm));
-    const char *la = std::getenv("PMDD_BIG_LEX_MAX_ARCS");
-    if (la && *la) lex_max_arcs_ = std::max(0, std::min(std::atoi(la), dev::kBigLexMaxArcs));
     const char *tw = std::getenv("PMDD_TILE_WINDOW_MAX");
     if (tw && *tw) window_max_fixed_ = std::atoll(tw);
     const char *pm = std::getenv("PMDD_LEX_PAIR_MAX");
@@ -1287,7 +1285,7 @@ int Engine::step() {
         int64_t tiles;
         size_t big_first, big_count;
         int64_t max_big;
-        int32_t max_big_arcs;      // most arcs of an oversized destination (merge rounds)
+        int32_t max_big_arcs;      // most arcs of an oversized destination
         int64_t items;             // destinations over the group's jobs
         int64_t big_passes;        // scratch passes of the oversized path
         int64_t big_rows;          // oversized candidate rows over the group's jobs (flat space)
@@ -1342,8 +1340,6 @@ int Engine::step() {
                 J.prev_sorted = s.sorted;
                 J.out_sorted = e.out_sorted;
                 J.pair_max = pair_max_for(I.d, I.opts.problem_type);
-                J.lex_big = (I.d == 3 && lex_tiles_) ? 1 : 0;
-                J.lex_max_arcs = lex_max_arcs_;
                 J.tile_base = gl.tiles;
                 tile_bases[pos] = gl.tiles;
                 item_bases[pos] = gl.items;
@@ -1940,8 +1936,6 @@ int Engine::step() {
                 J.tile_first = c.size[b] + J.num_items;
                 J.big_list = j == 1 ? new_big[c.count_idx] : c.big[pb];
                 J.pair_max = pair_max_for(I.d, I.opts.problem_type);
-                J.lex_big = (I.d == 3 && lex_tiles_) ? 1 : 0;
-                J.lex_max_arcs = lex_max_arcs_;
                 g.items[j] += J.num_items;
                 g.tiles[j] += c.ntiles;
                 const int y = nl + c.dir;  // the layer after it in this direction
@@ -2120,8 +2114,6 @@ int Engine::step() {
         L.total = gl.big_rows;
         L.sms = sms_;
         L.with_sfs = with_sfs(gl);
-        L.lex_big = gl.d == 3 && lex_tiles_;
-        L.lex_rounds = L.lex_big ? dev::lex_merge_rounds(std::min(gl.max_big_arcs, lex_max_arcs_)) : 0;
         L.mark_cap = static_cast<int>(std::min<int64_t>(gl.mark_cap, static_cast<int64_t>(gl.big_count)));
         L.plan = nullptr;
         // more SFS blocks than fit the SMs at once: start the largest destinations first
@@ -2131,8 +2123,7 @@ int Engine::step() {
         for (int64_t pass = 0; pass < gl.big_passes; ++pass) {
             L.pass = pass;
             if (!cuda_ok(dev::launch_big(gl.d, gl.wide, L, stream_), "oversized-destination kernels")) return -1;
-            launches_ += 1 + (L.mark_cap > 0 ? 1 + dev::kMaximaLaunches : 0) + (L.with_sfs ? 1 + (ordered ? 1 : 0) : 0) +
-                         (L.lex_big ? 1 + L.lex_rounds : 0);
+            launches_ += 1 + (L.mark_cap > 0 ? 1 + dev::kMaximaLaunches : 0) + (L.with_sfs ? 1 + (ordered ? 1 : 0) : 0);
         }
     }
     if (!sdjobs.empty()) {

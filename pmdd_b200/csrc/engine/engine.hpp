@@ -361,10 +361,6 @@ class Engine {
     static constexpr int32_t kDefaultPairMax = 48;
     bool lex_tiles_ = true;
     bool lex_tiles_for(int d) const { return d == 3 && lex_tiles_; }
-    // Oversized three-objective destinations of at most this many arc runs, all from
-    // sorted frontiers, take the lexicographic path (big_lex.cu); the others the
-    // SFS / pivot-mark passes.  PMDD_BIG_LEX_MAX_ARCS, 0 .. kBigLexMaxArcs.
-    static constexpr int32_t kDefaultLexMaxArcs = 16;
     // Layer runs (run.cu): a request by method 1 at the root, or whose next layer has at most
     // kRunEnter candidates, goes on layer by layer in one launch: up to run_layers_ layers
     // (PMDD_RUN_LAYERS, 0: off) when nothing else is under way, else kRunShared, since the
@@ -392,7 +388,6 @@ class Engine {
     int64_t chain_max_requests_ = 128;
     int64_t chain_max_cand_ = int64_t(1) << 17;
     int64_t chained_layers_total_ = 0;  // layers expanded by chained steps (statistics)
-    int32_t lex_max_arcs_ = kDefaultLexMaxArcs;
     int32_t lex_pair_max_fixed_ = -1;
     std::map<std::pair<int, int>, int64_t> tuned_pair_max_;
     int32_t pair_max_for(int d, int problem_type) const;

@@ -13,9 +13,8 @@
 //   expand:  candidate = parent point + arc weight, in run order;
 //   merge:   each candidate's position in its destination's lexicographic order is its
 //            index in its run plus, per other run, a binary search for how many of that
-//            run's points come before it (equal points: the lower run first); a
-//            destination with a run from an unsorted parent counts the points before it
-//            instead;
+//            run's points come before it (equal points: the lower run first); the points of
+//            a run from an unsorted parent are counted one by one;
 //   filter:  a warp per chunk of 32 consecutive merged positions, whatever destinations
 //            they belong to.  First every candidate against the 32 of its chunk (bit masks
 //            of the ones >= it in objective 1, and in both); a destination that goes on
@@ -41,8 +40,7 @@
 // 10-23): q is dropped iff another candidate p of the destination has p >= q on every
 // objective and (p != q or p comes first).  Of equal points the first in the merged order
 // stays; which copy stays does not change the frontier.  Oversized destinations are
-// left to big.cu, whose output is not in this order (out_sorted = 0): their children
-// merge by counting.
+// left to big.cu, whose output is not in this order (out_sorted = 0): its runs are counted.
 #pragma once
 
 #include "tile_pass.cuh"
@@ -143,7 +141,7 @@ __device__ __forceinline__ bool lex_items(LexSmem<T> &S, const ExpandJob &J, Run
             S.p0[q] = ld_point<RUN>(src) + static_cast<T>(w[0]);
             S.p1[q] = ld_point<RUN>(src + 1) + static_cast<T>(w[1]);
             S.p2[q] = ld_point<RUN>(src + 2) + static_cast<T>(w[2]);
-            I.item_of[q] = static_cast<uint16_t>(A.arc_item[x]);
+            I.item_of[q] = static_cast<uint16_t>(A.arc_item[x] & ~kUnsorted);
         }
         __syncthreads();
         clk.lap(3);
@@ -163,12 +161,14 @@ __device__ __forceinline__ bool lex_items(LexSmem<T> &S, const ExpandJob &J, Run
                 return tie;
             };
             int rank = 0;
-            if (I.item_count[k] == 0) {
-                rank = q - A.arc_pos[x];
-                const int y0 = I.item_arc0[k], y1 = I.item_arc0[k + 1];
-                for (int y = y0; y < y1; ++y) {
-                    if (y == x) continue;
-                    const int lo = A.arc_pos[y], hi = (y + 1 < y1) ? A.arc_pos[y + 1] : je;
+            const int y0 = I.item_arc0[k], y1 = I.item_arc0[k + 1];
+            for (int y = y0; y < y1; ++y) {
+                const int lo = A.arc_pos[y], hi = (y + 1 < y1) ? A.arc_pos[y + 1] : je;
+                if (A.arc_item[y] & kUnsorted) {  // a run in no order: count
+                    for (int j = lo; j < hi; ++j) rank += before(j, j < q) ? 1 : 0;
+                } else if (y == x) {
+                    rank += q - lo;
+                } else {
                     // points of run y before me: larger, or equal in a lower run; a prefix
                     int a = lo, b = hi;
                     while (a < b) {
@@ -178,8 +178,6 @@ __device__ __forceinline__ bool lex_items(LexSmem<T> &S, const ExpandJob &J, Run
                     }
                     rank += a - lo;
                 }
-            } else {
-                for (int j = js; j < je; ++j) rank += before(j, j < q) ? 1 : 0;
             }
             A.tag[q] = static_cast<int16_t>(js + rank);
         }

@@ -86,7 +86,7 @@ __device__ __forceinline__ bool pair_items(PairSmem<D, T> &S, const ExpandJob &J
             for (int o = 0; o < PackedPt<D, T>::kPad; ++o)
                 pt.v[o] = o < D ? ld_point<RUN>(src + (o < D ? o : 0)) + static_cast<T>(w[o < D ? o : 0]) : T(0);
             S.pts[q] = pt;
-            I.item_of[q] = static_cast<uint16_t>(A.arc_item[x]);
+            I.item_of[q] = static_cast<uint16_t>(A.arc_item[x] & ~kUnsorted);
         }
         __syncthreads();
         // --- filter

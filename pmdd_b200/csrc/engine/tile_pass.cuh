@@ -42,7 +42,6 @@ struct TileItems {
     int16_t item_arc0[kTileItemCap + 1]; // staged destination -> first staged arc
     int32_t item_a0g[kTileItemCap];      // staged destination -> first arc (global id)
     int64_t item_c0[kTileItemCap];       // staged destination -> job-local candidate start
-    uint8_t item_count[kTileItemCap];    // 1: a run from an unsorted parent
     int64_t warp_l[32], tot_l;           // scans
     int32_t warp_i[32];
     int32_t tot_i, tot_a;
@@ -50,10 +49,11 @@ struct TileItems {
 };
 
 // Their arcs.
+constexpr int16_t kUnsorted = 0x4000;    // the run's parent frontier is in no order
 struct TileArcs {
     int16_t tag[kTileCap];               // staged arc of each candidate
     int16_t arc_pos[kTileArcCap + 1];    // staged arc -> first candidate position
-    int16_t arc_item[kTileArcCap];       // staged arc -> staged destination
+    int16_t arc_item[kTileArcCap];       // staged arc -> staged destination, | kUnsorted
     int32_t arc_w[kTileArcCap];          // staged arc -> weight row
     int32_t arc_nbr[kTileArcCap];        // staged arc -> job-local neighbour (RUN: RunStage index)
 };
@@ -152,8 +152,7 @@ __device__ __forceinline__ int stage_items(TileItems &S, const ExpandJob &J, Run
             if (J.out_sorted) J.out_sorted[i] = (c == 0 || (resident && in_order)) ? 1 : 0;
             S.item_c0[k] = s;
             S.item_a0g[k] = a0;
-            S.item_count[k] = 0;
-            if (resident) {
+                if (resident) {
                 cnt[r] = static_cast<int32_t>(c);
                 narc[r] = a1 - a0;
             }
@@ -208,8 +207,8 @@ __device__ __forceinline__ int stage_items(TileItems &S, const ExpandJob &J, Run
     return n_it;
 }
 
-// Stages the arcs of the pass' n_it destinations and marks the ones with a run from an
-// unsorted parent; clears the tags.  A barrier must follow.
+// Stages the arcs of the pass' n_it destinations (marking runs from unsorted parents) and
+// clears the tags.  A barrier must follow.
 template <int NT, bool RUN>
 __device__ __forceinline__ void stage_arcs(TileItems &S, TileArcs &A, const ExpandJob &J, const RunStage *st, int n_it) {
     const int tid = threadIdx.x;
@@ -225,17 +224,18 @@ __device__ __forceinline__ void stage_arcs(TileItems &S, TileArcs &A, const Expa
         const int32_t a = S.item_a0g[k] + (x - S.item_arc0[k]);
         const int64_t c0 = J.arc_cand_off[a - J.arc_base];
         A.arc_pos[x] = static_cast<int16_t>(S.item_s[k] + (c0 - S.item_c0[k]));
-        A.arc_item[x] = static_cast<int16_t>(k);
+        bool sorted;
         if constexpr (RUN) {
             A.arc_nbr[x] = a - J.arc_base;
             A.arc_w[x] = st->w[a - J.arc_base];
-            if (st->sorted[a - J.arc_base] == 0) S.item_count[k] = 1;
+            sorted = st->sorted[a - J.arc_base] != 0;
         } else {
             const int32_t nb = J.arc_nbr[a] - J.prev_base;
             A.arc_nbr[x] = nb;
             A.arc_w[x] = J.arc_wrow[a];
-            if (J.prev_sorted == nullptr || J.prev_sorted[nb] == 0) S.item_count[k] = 1;
+            sorted = J.prev_sorted != nullptr && J.prev_sorted[nb] != 0;
         }
+        A.arc_item[x] = static_cast<int16_t>(sorted ? k : k | kUnsorted);
     }
     if (tid == 0) A.arc_pos[total_a] = static_cast<int16_t>(total);
     for (int q = tid; q < total; q += NT) A.tag[q] = -1;
