@@ -15,6 +15,7 @@ namespace dev {
 
 constexpr int kChunks = kTileCap / 32;
 constexpr unsigned kWarpAll = 0xffffffffu;
+constexpr int kSortRun = 32;
 
 template <bool RUN, typename V>
 __device__ __forceinline__ V ld_live(const V *p) {
@@ -45,7 +46,8 @@ struct TileItems {
     int64_t warp_l[32], tot_l;           // scans
     int32_t warp_i[32];
     int32_t tot_i, tot_a;
-    int32_t next_chunk, n_stair;
+    int32_t next_chunk, n_stair, n_sort;
+    int16_t sort_list[kTileCap / kSortRun];  // staged arcs whose runs are sorted first (lex_items.cuh)
 };
 
 // Their arcs.
@@ -202,6 +204,7 @@ __device__ __forceinline__ int stage_items(TileItems &S, const ExpandJob &J, Run
     if (tid == 0) {
         S.next_chunk = 0;
         S.n_stair = 0;
+        S.n_sort = 0;
     }
     __syncthreads();
     return n_it;
