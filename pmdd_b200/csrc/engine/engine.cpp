@@ -1082,9 +1082,13 @@ void Engine::plan_runs(std::vector<RunSlot> &runs) {
     for (auto &p : active_) {
         Instance &I = *p;
         if (I.phase == Instance::DONE) continue;
-        const Side &s = I.td;
-        const bool small = s.counted ? s.res.total <= kRunEnter && s.res.num_big == 0 : s.layer == 0;
-        bool ok = I.phase == Instance::RUNNING && I.opts.method == 1 && small && s.layer < I.L - 1;
+        const bool meet = I.opts.method == 3;
+        const Side &s = meet && I.td.score > I.bu.score ? I.bu : I.td;  // the side to expand
+        const bool end = s.layer == (&s == &I.td ? 0 : I.L - 1);
+        const bool small = s.counted ? s.res.total <= kRunEnter && s.res.num_big == 0 : end;
+        bool ok = I.phase == Instance::RUNNING && small;
+        if (meet) ok = ok && I.bu.layer - I.td.layer > 1 && I.opts.state_dominance <= 0;
+        else ok = ok && s.layer < I.L - 1;
         if (ok && I.run_skip > 0) {  // its last run stopped at once: a few ordinary steps first
             --I.run_skip;
             ok = false;
@@ -1097,8 +1101,11 @@ void Engine::plan_runs(std::vector<RunSlot> &runs) {
         RunSlot r;
         r.I = &I;
         r.sd = I.opts.state_dominance > 0 && I.sd_kind != 0 && I.sd_kind == I.opts.problem_type && I.d_sd_order;
-        r.last = static_cast<int32_t>(std::min<int64_t>(
-            I.L - 1, static_cast<int64_t>(I.td.layer) + (others ? std::min(run_layers_, kRunShared) : run_layers_)));
+        r.meet = I.opts.method == 3;
+        const int32_t most = others ? std::min(run_layers_, kRunShared) : run_layers_;
+        r.steps = most;
+        r.last = r.meet ? I.bu.layer - 1
+                        : static_cast<int32_t>(std::min<int64_t>(I.L - 1, static_cast<int64_t>(I.td.layer) + most));
         for (int l = I.td.layer + 1; l <= r.last; ++l) {
             r.vcap = std::max(r.vcap, I.nodes_in(l));
             r.max_arcs = std::max(r.max_arcs, I.arc_at_layer[l + 1] - I.arc_at_layer[l]);
@@ -1108,15 +1115,19 @@ void Engine::plan_runs(std::vector<RunSlot> &runs) {
             r.max_nodes = std::max(r.max_nodes, I.nodes_in(r.last + 1));
             r.max_arcs = std::max(r.max_arcs, I.arc_at_layer[r.last + 2] - I.arc_at_layer[r.last + 1]);
         }
+        if (r.meet) r.max_nodes = std::max(r.max_nodes, I.nodes_in(I.td.layer));
         r.vcap = static_cast<int32_t>(std::min<int64_t>(r.vcap, dev::kRunCap));
         r.pts_at = align256(sizeof(int64_t) * r.vcap) + align256((sizeof(int32_t) + 1) * static_cast<size_t>(r.vcap));
         const size_t bytes = r.pts_at + static_cast<size_t>(dev::kRunCap) * I.d * I.elem();
-        // two sets beside what is in use, with room to spare; else an ordinary step
-        if (arena_.used() + 4 * bytes > arena_.capacity()) continue;
-        r.buf[0] = static_cast<char *>(arena_.alloc(bytes));
-        r.buf[1] = r.buf[0] ? static_cast<char *>(arena_.alloc(bytes)) : nullptr;
-        if (!r.buf[1]) {
-            arena_.release(r.buf[0]);
+        // the sets beside what is in use, with room to spare; else an ordinary step
+        if (arena_.used() + 2 * r.sets() * bytes > arena_.capacity()) continue;
+        bool got = true;
+        for (int k = 0; k < r.sets() && got; ++k) {
+            r.buf[k] = static_cast<char *>(arena_.alloc(bytes));
+            got = r.buf[k] != nullptr;
+        }
+        if (!got) {
+            release_run(r);
             continue;
         }
         I.in_run = true;
@@ -1176,12 +1187,6 @@ int Engine::step() {
         }
         counters_.admitted++;
         reserved += std::max<int64_t>(0, pred - current_bytes(I));
-        if (I.phase == Instance::RUNNING) {
-            if (I.opts.method == 3) {
-                counts.push_back({&I, true, false});
-                counts.push_back({&I, false, false});
-            }  // method 1: a layer run from the root, or its count, below
-        }
         active_.push_back(std::move(*it));
         it = queued_.erase(it);
     }
@@ -1189,14 +1194,15 @@ int Engine::step() {
     counters_.queued_peak = std::max<int64_t>(counters_.queued_peak, static_cast<int64_t>(queued_.size()));
 
     // ------------------------------------------------------------ layer runs
-    // Requests by method 1 at the root, or whose next layer is small, run on from there in
-    // one launch (run.cu) instead of expanding one layer.
+    // Requests just admitted, or whose next layer is small, run on from there in one launch
+    // (run.cu) instead of expanding one layer; the others just admitted are counted.
     std::vector<RunSlot> runs;
     plan_runs(runs);
     for (auto &p : active_) {
         Instance &I = *p;
-        if (I.phase == Instance::RUNNING && I.opts.method == 1 && I.td.layer == 0 && !I.td.counted && !I.in_run)
-            counts.push_back({&I, true, false});
+        if (I.phase != Instance::RUNNING || I.in_run) continue;
+        if (I.td.layer == 0 && !I.td.counted) counts.push_back({&I, true, false});
+        if (I.opts.method == 3 && I.bu.layer == I.L - 1 && !I.bu.counted) counts.push_back({&I, false, false});
     }
 
     // ------------------------------------------------------------ expansions
@@ -1459,7 +1465,10 @@ int Engine::step() {
     for (RunSlot &r : runs) {
         r.count_idx = counts.size();
         counts.push_back({r.I, true, false});
+        if (r.meet) counts.push_back({r.I, false, false});
     }
+    std::vector<const RunSlot *> run_of_count;  // from first_run_count on
+    for (const RunSlot &r : runs) run_of_count.insert(run_of_count.end(), r.meet ? 2 : 1, &r);
     std::vector<dev::CountJob> cjobs(counts.size());
     std::vector<int64_t *> new_arc_off(counts.size(), nullptr);
     std::vector<int64_t *> new_big(counts.size(), nullptr);
@@ -1526,11 +1535,11 @@ int Engine::step() {
         Instance &I = *counts[k].I;
         const bool td = counts[k].td;
         if (k >= first_run_count) {  // sized for any layer the run may stop at
-            const RunSlot &r = runs[k - first_run_count];
+            const RunSlot &r = *run_of_count[k - first_run_count];
             dev::CountJob &J = cjobs[k];
             std::memset(&J, 0, sizeof(J));
-            J.item_arc_off = I.d_in_off;
-            J.arc_nbr = I.d_arc_src;
+            J.item_arc_off = td ? I.d_in_off : I.d_out_off;
+            J.arc_nbr = td ? I.d_arc_src : I.d_out_head;
             const size_t arc_bytes = align256(sizeof(int64_t) * (static_cast<size_t>(r.max_arcs) + 1));
             char *cb = static_cast<char *>(arena_.alloc(arc_bytes + sizeof(int64_t) * 2 * std::max(1, r.max_nodes)));
             new_arc_off[k] = reinterpret_cast<int64_t *>(cb);
@@ -1712,7 +1721,8 @@ int Engine::step() {
     // layer runs: descriptors staged by (objectives, point type); per run what the host reads
     // back (zeroed) and keep flags
     std::sort(runs.begin(), runs.end(), [](const RunSlot &a, const RunSlot &b) {
-        return std::make_tuple(a.I->d, a.I->wide, a.count_idx) < std::make_tuple(b.I->d, b.I->wide, b.count_idx);
+        return std::make_tuple(a.I->d, a.I->wide, a.meet, a.count_idx) <
+               std::make_tuple(b.I->d, b.I->wide, b.meet, b.count_idx);
     });
     const size_t st_run = align256(stage_bytes);
     if (!runs.empty()) stage_bytes = st_run + sizeof(dev::RunJob) * runs.size();
@@ -1821,24 +1831,32 @@ int Engine::step() {
         Instance &I = *r.I;
         dev::RunJob J;
         std::memset(&J, 0, sizeof(J));
-        J.item_arc_off = I.d_in_off;
-        J.arc_nbr = I.d_arc_src;
-        J.arc_wrow = I.d_arc_w;
+        auto side = [&](dev::RunSide &d, const Side &f, const int32_t *off, const int32_t *nbr, const int32_t *wrow,
+                        int set, size_t count) {
+            d.item_arc_off = off;
+            d.arc_nbr = nbr;
+            d.arc_wrow = wrow;
+            d.pts = f.pts;
+            d.off = f.off;
+            d.size = f.size;
+            d.sorted = f.sorted;
+            d.layer = f.layer;
+            d.score = f.score;
+            for (int b = 0; b < 2; ++b) {
+                d.b_off[b] = reinterpret_cast<int64_t *>(r.buf[set + b]);
+                d.b_size[b] = r.size(set + b);
+                d.b_sorted[b] = r.sorted(set + b);
+                d.b_pts[b] = r.pts(set + b);
+            }
+            d.count = reinterpret_cast<dev::CountJob *>(d_stage + off_c) + count;
+        };
+        side(J.td, I.td, I.d_in_off, I.d_arc_src, I.d_arc_w, 0, r.count_idx);
+        if (r.meet) side(J.bu, I.bu, I.d_out_off, I.d_out_head, I.d_out_w, 2, r.count_idx + 1);
         J.weights = I.d_weights;
         J.layer_off = I.d_layer_off;
-        J.pts = I.td.pts;
-        J.off = I.td.off;
-        J.size = I.td.size;
-        J.sorted = I.td.sorted;
-        J.layer = I.td.layer;
         J.last = r.last;
         J.terminal = I.L - 1;
-        for (int b = 0; b < 2; ++b) {
-            J.b_off[b] = reinterpret_cast<int64_t *>(r.buf[b]);
-            J.b_size[b] = r.size(b);
-            J.b_sorted[b] = r.sorted(b);
-            J.b_pts[b] = r.pts(b);
-        }
+        J.steps = r.steps;
         J.vcap = r.vcap;
         J.pair_max = pair_max_for(I.d, I.opts.problem_type);
         if (r.sd) {
@@ -1850,7 +1868,6 @@ int Engine::step() {
             J.keep = reinterpret_cast<uint8_t *>(d_run + r.at_keep);
         }
         J.out = reinterpret_cast<dev::RunOut *>(d_run) + k;
-        J.count = reinterpret_cast<dev::CountJob *>(d_stage + off_c) + r.count_idx;
         J.err = d_err_step;
         std::memcpy(hs + st_run + sizeof(dev::RunJob) * k, &J, sizeof(J));
     }
@@ -2089,9 +2106,11 @@ int Engine::step() {
         cudaMemsetAsync(d_run, 0, run_out_bytes, stream_);
         for (size_t i = 0; i < runs.size();) {
             size_t j = i + 1;
-            while (j < runs.size() && runs[j].I->d == runs[i].I->d && runs[j].I->wide == runs[i].I->wide) ++j;
+            while (j < runs.size() && runs[j].I->d == runs[i].I->d && runs[j].I->wide == runs[i].I->wide &&
+                   runs[j].meet == runs[i].meet)
+                ++j;
             if (!cuda_ok(dev::launch_layer_runs(runs[i].I->d, runs[i].I->wide, lex_tiles_for(runs[i].I->d),
-                                                reinterpret_cast<const dev::RunJob *>(d_stage + st_run) + i,
+                                                runs[i].meet, reinterpret_cast<const dev::RunJob *>(d_stage + st_run) + i,
                                                 static_cast<int>(j - i), stream_),
                          "run_layers_kernel"))
                 return -1;
@@ -2368,49 +2387,62 @@ int Engine::step() {
         Instance &I = *r.I;
         I.in_run = false;
         const dev::RunOut &o = reinterpret_cast<const dev::RunOut *>(hsum + s_run)[k];
-        int64_t *arc_off = new_arc_off[r.count_idx], *big = new_big[r.count_idx];
         if (I.phase != Instance::RUNNING) {  // cancelled or failed
             release_run(r);
-            arena_.release(arc_off);
+            for (size_t c = r.count_idx; c < r.count_idx + (r.meet ? 2 : 1); ++c) arena_.release(new_arc_off[c]);
             continue;
         }
-        Side &s = I.td;
         I.stats.kernel_expand_td_s += ms_expand * 1e-3;
         I.stats.kernel_total_s += (ms_expand + ms_rest) * 1e-3;
-        run_layers += o.done;
-        I.run_skip = o.done == 0 ? kRunSkip : 0;
-        arena_.release(s.arc_off);
-        arena_.release(s.big_list);
-        s.arc_off = nullptr;
-        s.big_list = nullptr;
-        if (o.done > 0) {
-            I.stats.work_candidates_total += o.cand_total;
-            I.stats.work_candidates_peak = std::max(I.stats.work_candidates_peak, o.cand_peak);
-            I.peak_cand = std::max(I.peak_cand, o.cand_peak);
-            I.stats.work_tile_candidates_total += o.cand_total;
-            I.stats.work_tile_survivors_total += o.tile_surv;
-            I.stats.work_stair_candidates_total += o.stair;
-            I.stats.work_frontier_survivors_total += o.surv_total;
-            I.stats.work_frontier_peak_points = std::max(I.stats.work_frontier_peak_points, o.surv_peak);
-            I.stats.dominance_filtered_total += o.removed;
-            I.stats.layers_td += o.done;
-            I.stats.work_chained_layers += o.done;
-            arena_.release(s.pts);
-            arena_.release(s.off);
-            arena_.release(s.size);
-            const int b = o.done & 1;
-            arena_.release(r.buf[b ^ 1]);
-            s.off = reinterpret_cast<int64_t *>(r.buf[b]);
-            s.size = r.size(b);
-            s.sorted = r.sorted(b);
-            s.pts = r.pts(b);
-            s.layer += o.done;
-            s.slot_points = dev::kRunCap;
-        } else {
-            release_run(r);
+        const int32_t layers = o.done + o.done_bu;
+        run_layers += layers;
+        I.run_skip = layers == 0 ? kRunSkip : 0;
+        I.stats.work_candidates_total += o.cand_total;
+        I.stats.work_candidates_peak = std::max(I.stats.work_candidates_peak, o.cand_peak);
+        I.peak_cand = std::max(I.peak_cand, o.cand_peak);
+        I.stats.work_tile_candidates_total += o.cand_total;
+        I.stats.work_tile_survivors_total += o.tile_surv;
+        I.stats.work_stair_candidates_total += o.stair;
+        I.stats.work_frontier_survivors_total += o.surv_total;
+        I.stats.work_frontier_peak_points = std::max(I.stats.work_frontier_peak_points, o.surv_peak);
+        I.stats.dominance_filtered_total += o.removed;
+        I.stats.layers_td += o.done;
+        I.stats.layers_bu += o.done_bu;
+        I.stats.work_chained_layers += layers;
+        for (int side = 0; side < (r.meet ? 2 : 1); ++side) {
+            Side &s = side == 0 ? I.td : I.bu;
+            const int32_t done = side == 0 ? o.done : o.done_bu;
+            const size_t c = r.count_idx + side;
+            const int set = 2 * side + (done & 1);  // the set the last layer was written to
+            arena_.release(s.arc_off);
+            arena_.release(s.big_list);
+            arena_.release(r.buf[set ^ 1]);
+            if (done > 0) {
+                arena_.release(s.pts);
+                arena_.release(s.off);
+                arena_.release(s.size);
+                s.off = reinterpret_cast<int64_t *>(r.buf[set]);
+                s.size = r.size(set);
+                s.sorted = r.sorted(set);
+                s.pts = r.pts(set);
+                s.layer += side == 0 ? done : -done;
+                s.slot_points = dev::kRunCap;
+            } else {
+                arena_.release(r.buf[set]);
+            }
+            s.arc_off = new_arc_off[c];
+            s.big_list = new_big[c];
+            s.res = hres[c];
+            s.counted = true;
+            if (done > 0 || I.opts.method == 1)
+                s.score = side == 0 ? s.res.total : static_cast<int64_t>(1.5 * static_cast<double>(s.res.total));
         }
-        if (s.layer == I.L - 1) {
-            arena_.release(arc_off);
+        if (r.meet) continue;
+        if (I.td.layer == I.L - 1) {  // the terminal: its frontier is the result
+            Side &s = I.td;
+            arena_.release(s.arc_off);
+            s.arc_off = nullptr;
+            s.big_list = nullptr;
             s.counted = false;
             I.result_n = o.final_size;
             I.result.resize(static_cast<size_t>(o.final_size) * I.d * I.elem());
@@ -2418,16 +2450,9 @@ int Engine::step() {
             I.stats.work_frontier_survivors_total += o.final_size;
             I.stats.work_frontier_peak_points = std::max<int64_t>(I.stats.work_frontier_peak_points, o.final_size);
             I.phase = Instance::DONE;
-        } else {
-            s.arc_off = arc_off;
-            s.big_list = big;
-            s.res = hres[r.count_idx];
-            s.counted = true;
-            s.score = s.res.total;
-            if (o.done > 0) {
-                I.stats.work_frontier_survivors_total += s.res.cur_total;
-                I.stats.work_frontier_peak_points = std::max(I.stats.work_frontier_peak_points, s.res.cur_total);
-            }
+        } else if (o.done > 0) {
+            I.stats.work_frontier_survivors_total += I.td.res.cur_total;
+            I.stats.work_frontier_peak_points = std::max(I.stats.work_frontier_peak_points, I.td.res.cur_total);
         }
     }
     chained_layers_total_ += run_layers;

@@ -166,17 +166,21 @@ struct Instance {
     int32_t nodes_in(int l) const { return layer_off[l + 1] - layer_off[l]; }
 };
 
-// A request's layer run in one step (run.cu).  Two buffer sets, each one block: slot offsets |
-// sizes and sorted flags | points.
+// A request's layer run in one step (run.cu).  Two buffer sets per side, each one block: slot
+// offsets | sizes and sorted flags | points.
 struct RunSlot {
     Instance *I = nullptr;
-    size_t count_idx = 0;               // the step's count of the layer it stops before
-    int32_t last = 0;                   // the last layer it may reach
+    bool meet = false;                  // method 3: both sides
+    size_t count_idx = 0;               // the step's count of the layer it stops before (method 3:
+                                        // top-down; the next index: bottom-up)
+    int32_t last = 0;                   // method 1: the last layer it may reach
+    int32_t steps = 0;                  // method 3: most layers
     bool sd = false;                    // with state dominance
     int32_t vcap = 0;                   // nodes of a layer the buffers hold
     int32_t max_nodes = 0, max_arcs = 0;  // of a layer the count may see
     size_t pts_at = 0, at_keep = 0;
-    char *buf[2] = {nullptr, nullptr};
+    char *buf[4] = {nullptr, nullptr, nullptr, nullptr};  // top-down sets, bottom-up sets
+    int sets() const { return meet ? 4 : 2; }
     int32_t *size(int b) const {
         return reinterpret_cast<int32_t *>(buf[b] + (sizeof(int64_t) * static_cast<size_t>(vcap) + 255) / 256 * 256);
     }
@@ -361,8 +365,9 @@ class Engine {
     static constexpr int32_t kDefaultPairMax = 48;
     bool lex_tiles_ = true;
     bool lex_tiles_for(int d) const { return d == 3 && lex_tiles_; }
-    // Layer runs (run.cu): a request by method 1 at the root, or whose next layer has at most
-    // kRunEnter candidates, goes on layer by layer in one launch: up to run_layers_ layers
+    // Layer runs (run.cu): a request at the root (method 3: at both ends), or whose next layer
+    // has at most kRunEnter candidates, goes on layer by layer in one launch (method 3: by
+    // the side rule, without state dominance): up to run_layers_ layers
     // (PMDD_RUN_LAYERS, 0: off) when nothing else is under way, else kRunShared, since the
     // others wait for the step.  A run that stops at once is not tried again for kRunSkip
     // steps.  With more than kRunMaxRequests requests (one cluster of 8 per 8 SMs) the

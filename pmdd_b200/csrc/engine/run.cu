@@ -72,8 +72,108 @@ struct RunSmem {
 
 // A layer's share of one block: destinations [v0, v1) and their arcs [a0, a1).
 struct RunShare {
-    int32_t x0, y0, nodes, v0, v1, a0, a1;
+    int32_t y0, nodes, v0, v1, a0, a1;
 };
+
+// The frontier a side expands from after `done` layers of the run.
+struct RunFrom {
+    const void *pts;
+    const int64_t *off;
+    const int32_t *size;
+    const uint8_t *sorted;
+};
+__device__ __forceinline__ RunFrom run_from(const RunSide &d, int done) {
+    if (done == 0) return {d.pts, d.off, d.size, d.sorted};
+    const int b = done & 1;
+    return {d.b_pts[b], d.b_off[b], d.b_size[b], d.b_sorted[b]};
+}
+
+// The block's share of layer y, expanded from layer x, with its arcs' neighbours and weight
+// rows fetched (as many as fit).
+__device__ __forceinline__ RunShare run_fetch(RunStage &st, const RunSide &d, const int32_t *layer_off, int x, int y,
+                                              int rank) {
+    RunShare h;
+    const int32_t x0 = layer_off[x];
+    h.y0 = layer_off[y];
+    h.nodes = layer_off[y + 1] - h.y0;
+    h.v0 = static_cast<int32_t>(static_cast<int64_t>(h.nodes) * rank / kRunBlocks);
+    h.v1 = static_cast<int32_t>(static_cast<int64_t>(h.nodes) * (rank + 1) / kRunBlocks);
+    h.a0 = d.item_arc_off[h.y0 + h.v0];
+    h.a1 = d.item_arc_off[h.y0 + h.v1];
+    for (int32_t k = threadIdx.x; k < min(h.a1 - h.a0, kRunRegion); k += kRunThreads) {
+        st.nbr[k] = d.arc_nbr[h.a0 + k] - x0;
+        st.w[k] = d.arc_wrow[h.a0 + k];
+    }
+    for (int32_t i = h.v0 + threadIdx.x; i <= h.v1; i += kRunThreads)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(d.item_arc_off + h.y0 + i));
+    return h;
+}
+
+// Candidate offsets of the block's arcs within its region, their parents' slots and order;
+// returns the candidates.  After run_fetch and a barrier; ends with a barrier.
+__device__ __forceinline__ int64_t run_gather(RunStage &st, const RunFrom &from, int32_t arcs, int64_t region,
+                                              int64_t *warp_l, int64_t *tot) {
+    constexpr int PER = kRunRegion / kRunThreads;
+    int32_t c[PER];
+    int64_t mine = 0;
+#pragma unroll
+    for (int r = 0; r < PER; ++r) {
+        const int k = threadIdx.x * PER + r;
+        c[r] = 0;
+        if (k < arcs) {
+            const int32_t nb = st.nbr[k];
+            c[r] = ld_live<true>(from.size + nb);
+            st.src[k] = ld_live64<true>(from.off + nb);
+            st.sorted[k] = ld_live<true>(reinterpret_cast<const unsigned char *>(from.sorted) + nb);
+        }
+        mine += c[r];
+    }
+    int64_t at = region + block_exclusive_scan<int64_t, kRunThreads>(mine, warp_l, tot);
+    const int64_t cand = *tot;
+#pragma unroll
+    for (int r = 0; r < PER; ++r) {
+        const int k = threadIdx.x * PER + r;
+        if (k < arcs) st.off[k] = at;
+        at += c[r];
+    }
+    if (threadIdx.x == 0) st.off[arcs] = region + cand;
+    __syncthreads();
+    return cand;
+}
+
+// The expansion of a share into buffer set b (one thread calls it).
+__device__ __forceinline__ void run_describe(ExpandJob &J, const RunJob &R, const RunSide &d, const RunShare &h,
+                                             const void *prev_pts, RunStage &st, int b, unsigned long long *tile) {
+    J.item_arc_off = d.item_arc_off;
+    J.weights = R.weights;
+    J.arc_cand_off = st.off;
+    J.arc_base = h.a0;
+    J.item_base = h.y0;
+    J.num_items = h.nodes;
+    J.prev_pts = prev_pts;
+    J.out_pts = d.b_pts[b];
+    J.out_off = d.b_off[b];
+    J.out_size = d.b_size[b];
+    J.out_sorted = d.b_sorted[b];
+    J.err = R.err;
+    J.tile_surv = tile;
+    J.pair_max = R.pair_max;
+    J.phase_clk = nullptr;
+    tile[0] = tile[1] = 0;
+    st.over = 0;
+}
+
+// Completes the count job of the layer y after layer x (y outside the DD: nothing to count).
+__device__ __forceinline__ void run_count_job(CountJob &C, const RunSide &d, const int32_t *layer_off, int x, int y,
+                                              bool more, const int32_t *x_size) {
+    C.cur_base = layer_off[x];
+    C.cur_nodes = more ? layer_off[x + 1] - layer_off[x] : 0;
+    C.cur_size = x_size;
+    C.item_base = more ? layer_off[y] : 0;
+    C.num_items = more ? layer_off[y + 1] - layer_off[y] : 0;
+    C.arc_base = more ? d.item_arc_off[layer_off[y]] : 0;
+    C.num_arcs = more ? d.item_arc_off[layer_off[y + 1]] - C.arc_base : 0;
+}
 
 }  // namespace
 
@@ -86,91 +186,28 @@ __global__ void __cluster_dims__(kRunBlocks, 1, 1) __launch_bounds__(kRunThreads
     RunStage &st = S.st;
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     const RunJob &R = jobs[blockIdx.x / kRunBlocks];
+    const RunSide &d = R.td;
     const int rank = static_cast<int>(blockIdx.x % kRunBlocks);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t region = static_cast<int64_t>(rank) * kRunRegion;
-    // the share of layer y, with its arcs' neighbours and weight rows fetched (as many as fit)
-    auto fetch = [&](int y) -> RunShare {
-        RunShare h;
-        h.x0 = R.layer_off[y - 1];
-        h.y0 = R.layer_off[y];
-        h.nodes = R.layer_off[y + 1] - h.y0;
-        h.v0 = static_cast<int32_t>(static_cast<int64_t>(h.nodes) * rank / kRunBlocks);
-        h.v1 = static_cast<int32_t>(static_cast<int64_t>(h.nodes) * (rank + 1) / kRunBlocks);
-        h.a0 = R.item_arc_off[h.y0 + h.v0];
-        h.a1 = R.item_arc_off[h.y0 + h.v1];
-        for (int32_t k = tid; k < min(h.a1 - h.a0, kRunRegion); k += NT) {
-            st.nbr[k] = R.arc_nbr[h.a0 + k] - h.x0;
-            st.w[k] = R.arc_wrow[h.a0 + k];
-        }
-        for (int32_t i = h.v0 + tid; i <= h.v1; i += NT)
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(R.item_arc_off + h.y0 + i));
-        return h;
-    };
     int done = 0;
     int64_t removed_total = 0, before_surv = 0;
     unsigned long long tile_surv = 0, stair = 0;
     int64_t cand_total = 0, cand_peak = 0, surv_total = 0, surv_peak = 0;
     if (tid == 0) S.removed = 0;
-    RunShare h = fetch(R.layer + 1);
+    RunShare h = run_fetch(st, d, R.layer_off, d.layer, d.layer + 1, rank);
     cluster.sync();  // every block has started: its shared memory may be written to
-    for (int y = R.layer + 1; y <= R.last; ++y) {
-        const int b = (y - R.layer) & 1;
-        const int64_t *x_off = done == 0 ? R.off : R.b_off[b ^ 1];
-        const int32_t *x_size = done == 0 ? R.size : R.b_size[b ^ 1];
-        const uint8_t *x_sorted = done == 0 ? R.sorted : R.b_sorted[b ^ 1];
+    for (int y = d.layer + 1; y <= R.last; ++y) {
+        const int b = (done + 1) & 1;
+        const RunFrom from = run_from(d, done);
         const int32_t arcs = h.a1 - h.a0;
         bool bad = h.nodes > R.vcap || arcs > kRunRegion;
-        if (tid == 0) {
-            S.tile[0] = S.tile[1] = 0;
-            st.over = 0;
-            ExpandJob &J = S.J;
-            J.item_arc_off = R.item_arc_off;
-            J.weights = R.weights;
-            J.arc_cand_off = st.off;
-            J.arc_base = h.a0;
-            J.item_base = h.y0;
-            J.num_items = h.nodes;
-            J.prev_pts = done == 0 ? R.pts : R.b_pts[b ^ 1];
-            J.out_pts = R.b_pts[b];
-            J.out_off = R.b_off[b];
-            J.out_size = R.b_size[b];
-            J.out_sorted = R.b_sorted[b];
-            J.err = R.err;
-            J.tile_surv = S.tile;
-            J.pair_max = R.pair_max;
-            J.phase_clk = nullptr;
-        }
+        if (tid == 0) run_describe(S.J, R, d, h, from.pts, st, b, S.tile);
         __syncthreads();
-        // --- candidate offsets of this block's arcs, within its region
         int64_t cand = 0;
         if (!bad) {
-            constexpr int PER = kRunRegion / NT;
-            int32_t c[PER];
-            int64_t mine = 0;
-#pragma unroll
-            for (int r = 0; r < PER; ++r) {
-                const int k = tid * PER + r;
-                c[r] = 0;
-                if (k < arcs) {
-                    const int32_t nb = st.nbr[k];
-                    c[r] = ld_live<true>(x_size + nb);
-                    st.src[k] = ld_live64<true>(x_off + nb);
-                    st.sorted[k] = ld_live<true>(reinterpret_cast<const unsigned char *>(x_sorted) + nb);
-                }
-                mine += c[r];
-            }
-            int64_t at = region + block_exclusive_scan<int64_t, NT>(mine, S.warp_l, &S.tot);
-            cand = S.tot;
-#pragma unroll
-            for (int r = 0; r < PER; ++r) {
-                const int k = tid * PER + r;
-                if (k < arcs) st.off[k] = at;
-                at += c[r];
-            }
-            if (tid == 0) st.off[arcs] = region + cand;
+            cand = run_gather(st, from, arcs, region, S.warp_l, &S.tot);
             bad = cand > kRunRegion;
-            __syncthreads();
         }
         // --- expand and filter
         if (!bad) {
@@ -188,7 +225,7 @@ __global__ void __cluster_dims__(kRunBlocks, 1, 1) __launch_bounds__(kRunThreads
         __syncwarp();
         auto token = cluster.barrier_arrive();
         const int32_t y0 = h.y0, nodes = h.nodes;
-        if (y < R.last) h = fetch(y + 1);
+        if (y < R.last) h = run_fetch(st, d, R.layer_off, y, y + 1, rank);
         cluster.barrier_wait(std::move(token));
         // --- does the layer stand?
         int64_t all_cand = 0, all_surv = 0, all_removed = 0, any_bad = 0;
@@ -220,12 +257,12 @@ __global__ void __cluster_dims__(kRunBlocks, 1, 1) __launch_bounds__(kRunThreads
                 sd.order = R.sd_order + y0;
                 sd.next = R.sd_kind == 2 ? R.sd_next + 2 * static_cast<int64_t>(y0) : nullptr;
                 sd.state = R.sd_state;
-                sd.in_off = R.item_arc_off;
-                sd.arc_src = R.arc_nbr;
-                sd.arc_w = R.arc_wrow;
-                sd.pts = R.b_pts[b];
-                sd.off = R.b_off[b];
-                sd.size = R.b_size[b];
+                sd.in_off = d.item_arc_off;
+                sd.arc_src = d.arc_nbr;
+                sd.arc_w = d.arc_wrow;
+                sd.pts = d.b_pts[b];
+                sd.off = d.b_off[b];
+                sd.size = d.b_size[b];
                 sd.keep = R.keep;
                 sd.removed = nullptr;
                 sd.node_base = y0;
@@ -252,7 +289,7 @@ __global__ void __cluster_dims__(kRunBlocks, 1, 1) __launch_bounds__(kRunThreads
         if (tile_surv) atomicAdd(reinterpret_cast<unsigned long long *>(&O.tile_surv), tile_surv);
         if (stair) atomicAdd(reinterpret_cast<unsigned long long *>(&O.stair), stair);
         // the last layer's removals were told to nobody when the run went to its end
-        const int64_t rest = R.layer + done == R.last ? S.removed : 0;
+        const int64_t rest = d.layer + done == R.last ? S.removed : 0;
         const int64_t all = rest + (rank == 0 ? removed_total : 0);
         if (all) atomicAdd(reinterpret_cast<unsigned long long *>(&O.removed), static_cast<unsigned long long>(all));
     }
@@ -262,43 +299,150 @@ __global__ void __cluster_dims__(kRunBlocks, 1, 1) __launch_bounds__(kRunThreads
         O.cand_peak = cand_peak;
         O.surv_total = surv_total;
         O.surv_peak = surv_peak;
-        const int x = R.layer + done, b = done & 1;
-        const int32_t *x_size = done == 0 ? R.size : R.b_size[b];
-        O.final_size = ld_live<true>(x_size);
-        O.final_off = ld_live64<true>(done == 0 ? R.off : R.b_off[b]);
-        CountJob &C = *R.count;
-        const bool more = x < R.terminal;  // a layer follows: its count
-        const int32_t x0 = R.layer_off[x], y0 = R.layer_off[x + 1];
-        C.cur_base = x0;
-        C.cur_nodes = more ? y0 - x0 : 0;
-        C.cur_size = x_size;
-        C.arc_base = more ? R.item_arc_off[y0] : 0;
-        C.num_arcs = more ? R.item_arc_off[R.layer_off[x + 2]] - C.arc_base : 0;
-        C.item_base = y0;
-        C.num_items = more ? R.layer_off[x + 2] - y0 : 0;
+        const int x = d.layer + done;
+        const RunFrom last = run_from(d, done);
+        O.final_size = ld_live<true>(last.size);
+        O.final_off = ld_live64<true>(last.off);
+        run_count_job(*d.count, d, R.layer_off, x, x + 1, x < R.terminal, last.size);
+    }
+}
+
+// Method 3: both sides, by the engine's rule.  The rule needs a side's next count, so a layer
+// meets twice: when it is written, and when the layer after it is counted (which also
+// gathers that layer's arcs, kept unless the other side goes next).
+template <int D, typename T, bool LEX>
+__global__ void __cluster_dims__(kRunBlocks, 1, 1) __launch_bounds__(kRunThreads, 1)
+    run_meet_kernel(const RunJob *__restrict__ jobs) {
+    constexpr int NT = kRunThreads;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    RunSmem<D, T, LEX> &S = *reinterpret_cast<RunSmem<D, T, LEX> *>(smem_raw);
+    RunStage &st = S.st;
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const RunJob &R = jobs[blockIdx.x / kRunBlocks];
+    const int rank = static_cast<int>(blockIdx.x % kRunBlocks);
+    const int tid = threadIdx.x;
+    const int64_t region = static_cast<int64_t>(rank) * kRunRegion;
+    int layer[2] = {R.td.layer, R.bu.layer}, done[2] = {0, 0};
+    int64_t score[2] = {R.td.score, R.bu.score};
+    unsigned long long tile_surv = 0, stair = 0;
+    int64_t cand_total = 0, cand_peak = 0, surv_total = 0, surv_peak = 0;
+    int staged = -1;  // the side whose next layer's arcs are gathered
+    int64_t cand = 0;
+    bool bad = false;
+    RunShare h{};
+    cluster.sync();  // every block has started: its shared memory may be written to
+    for (int step = 0; step < R.steps && layer[1] - layer[0] > 1; ++step) {
+        const int side = score[0] <= score[1] ? 0 : 1;
+        const RunSide &d = side == 0 ? R.td : R.bu;
+        const int dir = side == 0 ? 1 : -1;
+        const int b = (done[side] + 1) & 1;
+        const RunFrom from = run_from(d, done[side]);
+        if (staged != side) {
+            h = run_fetch(st, d, R.layer_off, layer[side], layer[side] + dir, rank);
+            bad = h.nodes > R.vcap || h.a1 - h.a0 > kRunRegion;
+            __syncthreads();
+            if (!bad) cand = run_gather(st, from, h.a1 - h.a0, region, S.warp_l, &S.tot);
+            bad |= cand > kRunRegion;
+        }
+        if (tid == 0) run_describe(S.J, R, d, h, from.pts, st, b, S.tile);
+        __syncthreads();
+        if (!bad) {
+            if constexpr (LEX) lex_items<T, NT, true>(S.items, S.J, &st, h.v0, h.v1, []() {});
+            else pair_items<D, T, NT, true>(S.items, S.J, &st, h.v0, h.v1, []() {});
+            bad = st.over != 0;
+        }
+        if (tid < kRunBlocks) {
+            RunPub *to = cluster.map_shared_rank(&S.pub[0][rank], tid);
+            to->cand = cand;
+            to->surv = static_cast<int64_t>(S.tile[0]);
+            to->bad = bad ? 1 : 0;
+        }
+        __syncwarp();
+        auto token = cluster.barrier_arrive();
+        const int next = layer[side] + 2 * dir;  // its next layer, if the sides stay apart
+        const bool count = layer[1] - layer[0] > 2;
+        if (count) h = run_fetch(st, d, R.layer_off, layer[side] + dir, next, rank);
+        cluster.barrier_wait(std::move(token));
+        int64_t all_cand = 0, all_surv = 0, any_bad = 0;
+#pragma unroll
+        for (int r = 0; r < kRunBlocks; ++r) {
+            all_cand += S.pub[0][r].cand;
+            all_surv += S.pub[0][r].surv;
+            any_bad |= S.pub[0][r].bad;
+        }
+        if (any_bad) break;  // every block of the cluster alike
+        cand_total += all_cand;
+        cand_peak = max(cand_peak, all_cand);
+        surv_total += all_surv;
+        surv_peak = max(surv_peak, all_surv);
+        tile_surv += S.tile[0];
+        stair += S.tile[1];
+        layer[side] += dir;
+        ++done[side];
+        if (!count) break;  // one layer apart
+        // --- the next layer's count on this side: its score
+        bad = h.nodes > R.vcap || h.a1 - h.a0 > kRunRegion;
+        __syncthreads();
+        cand = 0;
+        if (!bad) cand = run_gather(st, run_from(d, done[side]), h.a1 - h.a0, region, S.warp_l, &S.tot);
+        if (tid < kRunBlocks) {
+            RunPub *to = cluster.map_shared_rank(&S.pub[1][rank], tid);
+            to->cand = cand;
+            to->bad = bad ? 1 : 0;
+        }
+        cluster.sync();
+        int64_t total = 0;
+        any_bad = 0;
+#pragma unroll
+        for (int r = 0; r < kRunBlocks; ++r) {
+            total += S.pub[1][r].cand;
+            any_bad |= S.pub[1][r].bad;
+        }
+        if (any_bad) break;
+        bad = cand > kRunRegion;
+        score[side] = side == 0 ? total : static_cast<int64_t>(1.5 * static_cast<double>(total));
+        staged = side;
+    }
+    __syncthreads();
+    RunOut &O = *R.out;
+    if (tid == 0) {
+        if (tile_surv) atomicAdd(reinterpret_cast<unsigned long long *>(&O.tile_surv), tile_surv);
+        if (stair) atomicAdd(reinterpret_cast<unsigned long long *>(&O.stair), stair);
+    }
+    if (rank == 0 && tid == 0) {
+        O.done = done[0];
+        O.done_bu = done[1];
+        O.cand_total = cand_total;
+        O.cand_peak = cand_peak;
+        O.surv_total = surv_total;
+        O.surv_peak = surv_peak;
+        run_count_job(*R.td.count, R.td, R.layer_off, layer[0], layer[0] + 1, true, run_from(R.td, done[0]).size);
+        run_count_job(*R.bu.count, R.bu, R.layer_off, layer[1], layer[1] - 1, true, run_from(R.bu, done[1]).size);
     }
 }
 
 namespace {
 
 template <int D, typename T, bool LEX>
-cudaError_t launch_run_t(const RunJob *jobs, int num_jobs, cudaStream_t stream) {
+cudaError_t launch_run_t(bool meet, const RunJob *jobs, int num_jobs, cudaStream_t stream) {
     const size_t smem = sizeof(RunSmem<D, T, LEX>);
-    const cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(run_layers_kernel<D, T, LEX>), smem);
+    auto *kernel = meet ? run_meet_kernel<D, T, LEX> : run_layers_kernel<D, T, LEX>;
+    const cudaError_t e = ensure_smem_limit(reinterpret_cast<const void *>(kernel), smem);
     if (e != cudaSuccess) return e;
-    run_layers_kernel<D, T, LEX><<<static_cast<unsigned>(num_jobs) * kRunBlocks, kRunThreads, smem, stream>>>(jobs);
+    kernel<<<static_cast<unsigned>(num_jobs) * kRunBlocks, kRunThreads, smem, stream>>>(jobs);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_layer_runs(int d, bool wide, bool lex, const RunJob *jobs, int num_jobs, cudaStream_t stream) {
+cudaError_t launch_layer_runs(int d, bool wide, bool lex, bool meet, const RunJob *jobs, int num_jobs,
+                              cudaStream_t stream) {
     if (num_jobs <= 0) return cudaSuccess;
     if (lex && d == 3)
-        return wide ? launch_run_t<3, int64_t, true>(jobs, num_jobs, stream)
-                    : launch_run_t<3, int32_t, true>(jobs, num_jobs, stream);
-    if (wide) { PMDD_DISPATCH_D(d, (launch_run_t<DD, int64_t, false>(jobs, num_jobs, stream))); }
-    PMDD_DISPATCH_D(d, (launch_run_t<DD, int32_t, false>(jobs, num_jobs, stream)));
+        return wide ? launch_run_t<3, int64_t, true>(meet, jobs, num_jobs, stream)
+                    : launch_run_t<3, int32_t, true>(meet, jobs, num_jobs, stream);
+    if (wide) { PMDD_DISPATCH_D(d, (launch_run_t<DD, int64_t, false>(meet, jobs, num_jobs, stream))); }
+    PMDD_DISPATCH_D(d, (launch_run_t<DD, int32_t, false>(meet, jobs, num_jobs, stream)));
 }
 
 }  // namespace dev

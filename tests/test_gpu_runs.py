@@ -1,5 +1,5 @@
 """Layer runs (run.cu): small layers of a request followed in one launch give the frontiers
-and the work counters of the ordinary steps, whatever the run's length, for every
+and the work counters of the ordinary steps, by methods 1 and 3, whatever the run's length, for every
 objective count, int32 and int64 points, with state dominance, from host and resident
 DDs, and where a run stops at an oversized destination or a layer that outgrows a block."""
 import json
@@ -24,7 +24,8 @@ from conftest import frontier_digest
 from pmdd_b200 import instances as I
 KEYS = ("work_candidates_total", "work_candidates_peak", "work_frontier_survivors_total",
         "work_frontier_peak_points", "dominance_filtered_total", "layers_td",
-        "work_tile_candidates_total", "work_tile_survivors_total")
+        "work_tile_candidates_total", "work_tile_survivors_total", "layers_bu", "layer_coupling", "cutset_size",
+        "work_join_products_total")
 out = []
 def text(profits, weights, cap):
     rows = [f"{{profits.shape[1]}} 1 {{profits.shape[0]}}"] + [" ".join(map(str, r)) for r in profits]
@@ -45,11 +46,21 @@ for pt, t, d in ((1, I.knapsack_text(40, 3, 5), 3), (1, I.knapsack_text(24, 4, 6
                  (2, I.setpacking_text(60, 20, 4, 8), 4), (3, I.tsp_text(10, 3, 1), 3), (3, I.tsp_text(9, 5, 2), 5)):
     for sd in (0, 1):
         add(lambda st: [P.enumerate_dd(P.DecisionDiagram.from_text(t, pt, d), state_dominance=sd, stats=st)])
+        add(lambda st: [P.enumerate_dd(P.DecisionDiagram.from_text(t, pt, d), method=3, state_dominance=sd, stats=st)])
+for d in range(1, 9):
+    n = 30 if d < 5 else 20
+    add(lambda st: [P.enumerate_dd(P.DecisionDiagram.from_text(I.knapsack_text(n, d, 80 + d), 1, d), method=3, stats=st)])
+add(lambda st: [P.enumerate_dd(P.DecisionDiagram.from_text(text(p4.astype(np.int64) * 2_000_000, w4, c4), 1, 4), method=3,
+                               stats=st)])
+add(lambda st: [P.enumerate_dd(P.DecisionDiagram.from_text(I.tsp_text(3, 3, 1), 3, 3), method=3, stats=st)])
+add(lambda st: [P.enumerate_dd(P.DecisionDiagram.from_text(I.knapsack_text(2, 3, 1), 1, 3), method=3, stats=st)])
 res = P.ResidentSet.from_knapsack([I.knapsack_arrays(20 + i, 3, 60 + i) for i in range(5)])
 add(lambda st: res.enumerate(stats=st))
 add(lambda st: res.enumerate(state_dominance=1, stats=st))
 tsp = P.ResidentSet.from_tsp([I.tsp_arrays(8 + i, 3, i) for i in range(3)])
 add(lambda st: tsp.enumerate(stats=st))
+add(lambda st: tsp.enumerate(method=3, stats=st))
+add(lambda st: res.enumerate(method=3, stats=st))
 add(lambda st: P.enumerate_batch([P.DecisionDiagram.from_text(I.knapsack_text(20 + i, 3 + i % 3, i), 1, 3 + i % 3)
                                   for i in range(12)], stats=st))
 print(json.dumps(out))
