@@ -1630,7 +1630,9 @@ int Engine::step() {
             if (I.opts.method == 1 && !cp.td) continue;
             const int32_t ei = exp_index(I, cp.td);
             const ExpPlan *e = ei >= 0 ? &exps[ei] : nullptr;
-            if (e == nullptr || e->cand > chain_max_cand_) continue;
+            // (after a layer with oversized destinations the next one has some as a rule: a chain
+            // that stops there at once costs 40 us of launches)
+            if (e == nullptr || e->cand > chain_max_cand_ || e->num_big > 0) continue;
             if (I.chain_skip > 0) {  // its last chain went nowhere (method 3): wait a little
                 --I.chain_skip;
                 continue;
