@@ -202,23 +202,24 @@ static void setpacking_sd_layout(const pmdd_dd &dd, Instance *I) {
     const int32_t N = dd.num_nodes, W = dd.state_words, nb = dd.num_layers - 1;
     I->sd_order.assign(N, 0);
     I->sd_next.assign(2 * static_cast<size_t>(N), 0);
-    std::vector<int32_t> pc, first(nb + 1);
+    std::vector<int32_t> pc, first(nb + 1), at(static_cast<size_t>(nb) + 2);
     for (int l = 0; l < dd.num_layers; ++l) {
         const int32_t b = dd.layer_offsets[l], e = dd.layer_offsets[l + 1], cnt = e - b;
-        pc.assign(cnt, 0);
+        pc.resize(cnt);
+        std::fill(at.begin(), at.end(), 0);
         for (int32_t i = 0; i < cnt; ++i) {
             const uint64_t *s = dd.node_state + static_cast<size_t>(b + i) * W;
-            for (int32_t w = 0; w < W; ++w) pc[i] += __builtin_popcountll(s[w]);
+            int32_t c = 0;
+            for (int32_t w = 0; w < W; ++w) c += __builtin_popcountll(s[w]);
+            pc[i] = std::min(c, nb);
+            ++at[pc[i] + 1];
         }
+        // counting sort by size, ids ascending (sizes >= nb take no part: one bucket)
+        for (size_t k = 1; k < at.size(); ++k) at[k] += at[k - 1];
+        // first[k] = first order position with size >= k
+        for (int32_t k = 0; k <= nb; ++k) first[k] = at[k];
         int32_t *ord = I->sd_order.data() + b;
-        for (int32_t i = 0; i < cnt; ++i) ord[i] = i;
-        std::stable_sort(ord, ord + cnt, [&pc](int32_t x, int32_t y) { return pc[x] < pc[y]; });
-        // first[k] = first order position with size >= k (sizes >= nb take no part)
-        int32_t p = 0;
-        for (int32_t k = 0; k <= nb; ++k) {
-            while (p < cnt && pc[ord[p]] < k) ++p;
-            first[k] = p;
-        }
+        for (int32_t i = 0; i < cnt; ++i) ord[at[pc[i]]++] = i;
         int32_t *nx = I->sd_next.data() + 2 * static_cast<size_t>(b);
         for (int32_t k = 0; k + 1 < nb; ++k) {
             if (first[k + 1] - first[k] < 2) continue;
