@@ -1658,7 +1658,9 @@ int Engine::step() {
                 c.last = std::min<int32_t>(want, (cp.td ? o.layer - e->nl : e->nl - o.layer) - 1);
             }
             if (c.last <= 0) continue;
-            c.cap = std::min<int64_t>(std::max<int64_t>(8 * std::max<int64_t>(e->cand, 1), 16384), int64_t(1) << 22);
+            // room for layers 8 times as large while they are small, twice as large beyond
+            c.cap = std::max<int64_t>({16384, std::min<int64_t>(8 * std::max<int64_t>(e->cand, 1), 65536), 2 * e->cand});
+            c.cap = std::min<int64_t>(c.cap, int64_t(1) << 22);
             c.ntiles = c.cap / e->window + 2;
             for (int j = 1; j <= c.last; ++j) {
                 const int x = e->nl + c.dir * j;  // the layer chained layer j writes
