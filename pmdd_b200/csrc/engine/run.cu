@@ -19,10 +19,13 @@
 // Frontiers written by other blocks are read past the L1 cache (ld_live): the buffers
 // alternate, so a line of the layer before last may still be there.
 //
-// One B200, a layer: about 10 us, a chain of dependent loads, block barriers and the cluster's,
-// against 23 us for the two launches of a chained one.  KP d=3 n=20: 21 layers in 0.21 ms (call 0.77 -> 0.37 ms); set packing d=3 n=100: 1.1
-// ms (3.0 -> 1.27 ms); n=91 with state dominance, which ordinary steps take one layer at a
-// time: 2.7 ms (8.9 -> 5.1 ms).
+// One B200, a layer: about 10 us, a chain of dependent loads, block barriers and the
+// cluster's, against 23 us for the two launches of a chained one.  KP d=3 n=20: 21 layers
+// in 0.21 ms (call 0.77 -> 0.32 ms); set packing d=3 n=100: 1.1 ms (3.0 -> 1.27 ms); n=91
+// with state dominance, which ordinary steps take one layer at a time: 2.2 ms (8.9 -> 3.1
+// ms, of which 1.5 ms since the orders are counting-sorted at preparation; 2.7 ms before a
+// node's loads went out together, its partners' labels 32 at a time, and nodes that lose
+// no label were left out of the compaction).
 #include "run.cuh"
 
 #include <cooperative_groups.h>
@@ -272,11 +275,16 @@ __global__ void __cluster_dims__(kRunBlocks, 1, 1) __launch_bounds__(kRunThreads
             }
             __syncthreads();
             constexpr int kWarps = NT / 32;
-            for (int32_t n = rank * kWarps + warp; n < nodes; n += kRunBlocks * kWarps)
-                sd_mark_node<D, T, true>(S.sd, n, lane);
+            const int32_t p0 = rank * kWarps + warp;
+            uint64_t drops = 0;  // of the warp's nodes, the ones that lose a label (its 64th on: unknown)
+            int i = 0;
+            for (int32_t p = p0; p < nodes; p += kRunBlocks * kWarps, ++i)
+                if (sd_mark_node<D, T, true>(S.sd, p, lane) && i < 64) drops |= uint64_t(1) << i;
             cluster.sync();
-            for (int32_t n = rank * kWarps + warp; n < nodes; n += kRunBlocks * kWarps) {
-                const int32_t gone = sd_compact_node<D, T, true>(S.sd, n, lane);
+            i = 0;
+            for (int32_t p = p0; p < nodes; p += kRunBlocks * kWarps, ++i) {
+                if (i < 64 && !(drops >> i & 1)) continue;
+                const int32_t gone = sd_compact_node<D, T, true>(S.sd, S.sd.order[p], lane);
                 if (lane == 0 && gone > 0) atomicAdd(&S.removed, gone);
             }
             cluster.sync();

@@ -23,14 +23,27 @@ __device__ __forceinline__ int first_vertex(const uint64_t *s, int W) {
     return -1;
 }
 
-// Keep flags of the labels of the node at position `pos` of the layer's order.
+// Keep flags of the labels of the node at position `pos` of the layer's order; whether any
+// of them goes.  What a node needs is asked for at once, then waited for: one warp has one
+// node in a small layer, and its loads in a row are the time.
 template <int D, typename T, bool RUN>
-__device__ __forceinline__ void sd_mark_node(const StateDomJob &J, int32_t pos, int lane) {
+__device__ __forceinline__ bool sd_mark_node(const StateDomJob &J, int32_t pos, int lane) {
     const int32_t n1 = J.order[pos];
     const int32_t s1 = ld_live<RUN>(J.size + n1);
-    if (s1 == 0) return;
+    const int64_t o1 = ld_live64<RUN>(J.off + n1);
+    const int32_t b1 = J.in_off[J.node_base + n1], e1 = J.in_off[J.node_base + n1 + 1];
+    const int W = J.state_words;
+    const uint64_t *st1 = J.state + static_cast<int64_t>(J.node_base + n1) * W;
+    int32_t qb = 0, qe = 0;
+    uint64_t w0 = 0;
+    if (J.kind == 2) {
+        qb = J.next[2 * pos];
+        qe = J.next[2 * pos + 1];
+        w0 = st1[0];
+    }
+    if (s1 == 0) return false;
     // siblings under one single parent (through different arc types) are not compared
-    const int32_t a1 = single_in_arc(J, n1);
+    const int32_t a1 = e1 - b1 == 1 ? b1 : -1;
     auto skipped = [&](int32_t n2) -> bool {
         if (n2 < 0 || a1 < 0) return false;
         const int32_t a2 = single_in_arc(J, n2);
@@ -40,18 +53,17 @@ __device__ __forceinline__ void sd_mark_node(const StateDomJob &J, int32_t pos, 
     if (J.kind == 2) {
         // first node of the partner bucket with the same lowest vertex, not a
         // single-parent sibling, whose state contains n1's
-        const int32_t qb = J.next[2 * pos], qe = J.next[2 * pos + 1];
-        const int W = J.state_words;
-        const uint64_t *st1 = J.state + static_cast<int64_t>(J.node_base + n1) * W;
-        const int ff1 = first_vertex(st1, W);
+        const int ff1 = w0 != 0 ? __ffsll(static_cast<long long>(w0)) - 1 : first_vertex(st1, W);
         for (int32_t p = qb; p < qe && part0 < 0; p += 32) {
             const int32_t q = p + lane;
             bool ok = false;
             if (q < qe) {
                 const int32_t n2 = J.order[q];
                 const uint64_t *st2 = J.state + static_cast<int64_t>(J.node_base + n2) * W;
-                ok = first_vertex(st2, W) == ff1 && !skipped(n2);
-                for (int w = 0; w < W && ok; ++w) ok = (st1[w] & ~st2[w]) == 0;
+                ok = (w0 & ~st2[0]) == 0;
+                for (int w = 1; w < W; ++w) ok &= (st1[w] & ~st2[w]) == 0;
+                // few contain the state: the rest of the test is theirs alone
+                ok = ok && first_vertex(st2, W) == ff1 && !skipped(n2);
             }
             const unsigned m = __ballot_sync(kWarpAll, ok);
             if (m != 0) part0 = J.order[p + __ffs(m) - 1];
@@ -76,7 +88,7 @@ __device__ __forceinline__ void sd_mark_node(const StateDomJob &J, int32_t pos, 
         if (skipped(part1)) part1 = -1;
     }
     const T *P = static_cast<const T *>(J.pts);
-    const int64_t o1 = ld_live64<RUN>(J.off + n1);
+    bool drops = false;
     for (int32_t kb = 0; kb < s1; kb += 32) {
         const int32_t k = kb + lane;
         const bool valid = k < s1;
@@ -90,16 +102,24 @@ __device__ __forceinline__ void sd_mark_node(const StateDomJob &J, int32_t pos, 
             if (n2 < 0) continue;
             const int64_t o2 = ld_live64<RUN>(J.off + n2);
             const int32_t s2 = ld_live<RUN>(J.size + n2);
-            for (int32_t t = 0; t < s2; ++t) {
+            for (int32_t tb = 0; tb < s2; tb += 32) {
                 if (__all_sync(kWarpAll, dom)) break;
-                bool ge = true;
+                T y[D];
 #pragma unroll
-                for (int o = 0; o < D; ++o) ge &= (ld_point<RUN>(P + (o2 + t) * D + o) >= x[o]);
-                dom |= ge;
+                for (int o = 0; o < D; ++o) y[o] = tb + lane < s2 ? ld_point<RUN>(P + (o2 + tb + lane) * D + o) : T(0);
+                const int n = min(s2 - tb, 32);
+                for (int t = 0; t < n; ++t) {
+                    bool ge = true;
+#pragma unroll
+                    for (int o = 0; o < D; ++o) ge &= (__shfl_sync(kWarpAll, y[o], t) >= x[o]);
+                    dom |= ge;
+                }
             }
         }
         if (valid) J.keep[o1 + k] = dom ? 0 : 1;
+        drops |= __any_sync(kWarpAll, valid && dom);
     }
+    return drops;
 }
 
 // Packs the kept labels of node n to the front of its slot; returns how many went.
@@ -113,12 +133,14 @@ __device__ __forceinline__ int32_t sd_compact_node(const StateDomJob &J, int32_t
     for (int32_t kb = 0; kb < s; kb += 32) {
         const int32_t k = kb + lane;
         const bool keep = k < s && ld_live<RUN>(reinterpret_cast<const unsigned char *>(J.keep) + o + k) != 0;
+        const unsigned m = __ballot_sync(kWarpAll, keep);
+        const int32_t dst = kept + __popc(m & ((1u << lane) - 1u));
+        const bool moves = keep && dst != k;
         T x[D];
 #pragma unroll
-        for (int q = 0; q < D; ++q) x[q] = keep ? ld_point<RUN>(P + (o + k) * D + q) : T(0);
-        const unsigned m = __ballot_sync(kWarpAll, keep);  // every lane has loaded before any stores
-        const int32_t dst = kept + __popc(m & ((1u << lane) - 1u));
-        if (keep && dst != k) {
+        for (int q = 0; q < D; ++q) x[q] = moves ? ld_point<RUN>(P + (o + k) * D + q) : T(0);
+        __syncwarp();  // every lane has loaded before any stores
+        if (moves) {
 #pragma unroll
             for (int q = 0; q < D; ++q) P[(o + dst) * D + q] = x[q];
         }
