@@ -338,7 +338,7 @@ int64_t pmdd_launch_count(void);
  * engines read at start-up (PMDD_TUNING_FILE, else the per-user cache written by
  * pmdd_b200.autotune).  No counterpart in the reference, which has one filter path. */
 int64_t pmdd_tuned_mark_min(const char *path, int32_t nobjs, int32_t problem_type);
-/* The three-objective crossover between the pairwise check and the staircase warp
+/* The three-objective crossover between the pairwise check and the staircases
  * (destinations of at most this many candidates are checked pairwise) that the tuning
  * file holds for (nobjs, problem_type), or -1 if none (engines then use 48).  Same file
  * rules as pmdd_tuned_mark_min.  No counterpart in the reference, whose filter is

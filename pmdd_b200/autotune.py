@@ -18,7 +18,7 @@ without "big_mark_min" ({"builtin": true, ...}), which the engine reads as untun
 
 Three-objective families also get "lex_pair_max": in the lexicographic tiles,
 destinations of at most that many candidates are checked pairwise against the points
-before them and larger ones by a staircase warp.  It is timed over PAIR_MAX_SIZES with the
+before them and larger ones against staircases.  It is timed over PAIR_MAX_SIZES with the
 chosen oversized crossover in place (PMDD_LEX_PAIR_MAX in a fresh process); sizes within
 2 % of the fastest tie and the default (48) wins a tie, else the smallest.
 

@@ -93,7 +93,7 @@ struct ExpandJob {
     int64_t big_rows;              // scratch rows (candidates) one pass can use
     uint32_t *err;
     unsigned long long *tile_surv; // [0]: survivors written by the tile kernel, [1]: candidates of
-                                   // destinations filtered by staircase warps (both added to)
+                                   // destinations filtered by staircases (both added to)
     // Lexicographic order (three objectives): a node whose flag is 1 holds its frontier in
     // descending lexicographic order.  prev_sorted is indexed like prev_size; the tile
     // kernels write out_sorted for every destination they stage (1 only when they wrote
@@ -101,7 +101,7 @@ struct ExpandJob {
     const uint8_t *prev_sorted;
     uint8_t *out_sorted;
     int32_t pair_max;              // lexicographic tiles: destinations of at most this many
-                                   // candidates are checked pairwise, larger ones by a staircase warp
+                                   // candidates are checked pairwise, larger ones by staircases
     unsigned long long *phase_clk; // diagnostic: cycles per tile phase (lexicographic tiles), or nullptr
 };
 
