@@ -40,24 +40,6 @@ __device__ __forceinline__ V block_exclusive_scan(V x, V *warp_buf, V *total) {
     return r;
 }
 
-__device__ __forceinline__ int warp_min_i(int x) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x = min(x, __shfl_xor_sync(0xffffffffu, x, o));
-    return x;
-}
-
-__device__ __forceinline__ int warp_max_i(int x) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x = max(x, __shfl_xor_sync(0xffffffffu, x, o));
-    return x;
-}
-
-__device__ __forceinline__ int64_t warp_min_i64(int64_t x) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x = min(x, static_cast<int64_t>(__shfl_xor_sync(0xffffffffu, x, o)));
-    return x;
-}
-
 // A point padded to a 16-byte multiple so that a warp reads one candidate from shared
 // memory with vector loads that broadcast to all lanes.
 template <int D, typename T>
