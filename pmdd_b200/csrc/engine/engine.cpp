@@ -1067,16 +1067,18 @@ struct ChainGroup {
 std::atomic<int64_t> g_total_launches{0};
 
 void Engine::release_run(RunSlot &r) {
-    for (char *&b : r.buf) {
-        arena_.release(b);
-        b = nullptr;
-    }
+    for (char *b : r.buf) arena_.release(b);
+    for (char *c : r.cnt) arena_.release(c);
     r.I->in_run = false;
 }
 
 void Engine::plan_runs(std::vector<RunSlot> &runs) {
     for (auto &p : active_) p->in_run = false;
     if (run_layers_ <= 0 || chain_layers_ <= 0 || static_cast<int64_t>(active_.size()) > kRunMaxRequests) return;
+    if (run_hold_ > 0) {
+        --run_hold_;
+        return;
+    }
     // other requests wait for the step's runs: long ones only when nothing else is under way
     bool others = !queued_.empty();
     std::vector<Instance *> picked;
@@ -1097,6 +1099,8 @@ void Engine::plan_runs(std::vector<RunSlot> &runs) {
         if (ok) picked.push_back(&I);
         else others = true;
     }
+    const size_t room = (arena_.capacity() - std::min(arena_.used(), arena_.capacity())) / kRunRoom;
+    size_t taken = 0;
     for (Instance *p : picked) {
         Instance &I = *p;
         RunSlot r;
@@ -1119,18 +1123,26 @@ void Engine::plan_runs(std::vector<RunSlot> &runs) {
         if (r.meet) r.max_nodes = std::max(r.max_nodes, I.nodes_in(I.td.layer));
         r.vcap = static_cast<int32_t>(std::min<int64_t>(r.vcap, dev::kRunCap));
         r.pts_at = align256(sizeof(int64_t) * r.vcap) + align256((sizeof(int32_t) + 1) * static_cast<size_t>(r.vcap));
-        const size_t bytes = r.pts_at + static_cast<size_t>(dev::kRunCap) * I.d * I.elem();
-        // the sets beside what is in use, with room to spare; else an ordinary step
-        if (arena_.used() + 2 * r.sets() * bytes > arena_.capacity()) continue;
+        r.keep_at = r.pts_at + align256(static_cast<size_t>(dev::kRunCap) * I.d * I.elem());
+        const size_t bytes = r.keep_at + (r.sd ? static_cast<size_t>(dev::kRunCap) : 0);
+        r.arc_bytes = align256(sizeof(int64_t) * (static_cast<size_t>(r.max_arcs) + 1));
+        const size_t cnt_bytes = r.arc_bytes + sizeof(int64_t) * 2 * static_cast<size_t>(std::max(1, r.max_nodes));
+        const size_t need = r.sets() * bytes + r.sides() * cnt_bytes;
+        if (taken + need > room) continue;
         bool got = true;
         for (int k = 0; k < r.sets() && got; ++k) {
             r.buf[k] = static_cast<char *>(arena_.alloc(bytes));
             got = r.buf[k] != nullptr;
         }
+        for (int k = 0; k < r.sides() && got; ++k) {
+            r.cnt[k] = static_cast<char *>(arena_.alloc(cnt_bytes));
+            got = r.cnt[k] != nullptr;
+        }
         if (!got) {
             release_run(r);
             continue;
         }
+        taken += need;
         I.in_run = true;
         runs.push_back(r);
     }
@@ -1469,20 +1481,21 @@ int Engine::step() {
         if (r.meet) counts.push_back({r.I, false, false});
     }
     std::vector<const RunSlot *> run_of_count;  // from first_run_count on
-    for (const RunSlot &r : runs) run_of_count.insert(run_of_count.end(), r.meet ? 2 : 1, &r);
+    for (const RunSlot &r : runs) run_of_count.insert(run_of_count.end(), r.sides(), &r);
     std::vector<dev::CountJob> cjobs(counts.size());
     std::vector<int64_t *> new_arc_off(counts.size(), nullptr);
     std::vector<int64_t *> new_big(counts.size(), nullptr);
     // The step's summary block: everything the host reads back after the step, in one
     // device allocation and one copy: count results | tile survivors per expansion |
-    // labels removed by state dominance per job | error word.  All but the count
-    // results start at zero (one memset).
+    // labels removed by state dominance per job | error word | tile queues | what the layer
+    // runs did.  All but the count results start at zero (one memset).
     const size_t f_ts = sizeof(dev::CountResult) * counts.size();
     const size_t f_sd = f_ts + 2 * sizeof(unsigned long long) * exps.size();  // (survivors, staircase) per expansion
     const size_t f_err = f_sd + sizeof(int64_t) * sdjobs.size();
     const size_t f_clk = f_err + sizeof(uint64_t);  // PMDD_TRACE: tile phase cycles (8 counters)
     const size_t f_q = f_clk + (trace_ ? 8 * sizeof(unsigned long long) : 0);  // tile queue per group
-    const size_t f_total = f_q + sizeof(unsigned long long) * glaunch.size();
+    const size_t f_run = f_q + sizeof(unsigned long long) * glaunch.size();
+    const size_t f_total = f_run + sizeof(dev::RunOut) * runs.size();
     char *d_fixed = static_cast<char *>(scratch(f_total));
     dev::CountResult *d_results = counts.empty() ? nullptr : reinterpret_cast<dev::CountResult *>(d_fixed);
     unsigned long long *d_tile_surv = d_fixed ? reinterpret_cast<unsigned long long *>(d_fixed + f_ts) : nullptr;
@@ -1541,14 +1554,9 @@ int Engine::step() {
             std::memset(&J, 0, sizeof(J));
             J.item_arc_off = td ? I.d_in_off : I.d_out_off;
             J.arc_nbr = td ? I.d_arc_src : I.d_out_head;
-            const size_t arc_bytes = align256(sizeof(int64_t) * (static_cast<size_t>(r.max_arcs) + 1));
-            char *cb = static_cast<char *>(arena_.alloc(arc_bytes + sizeof(int64_t) * 2 * std::max(1, r.max_nodes)));
+            char *cb = r.cnt[k - r.count_idx];
             new_arc_off[k] = reinterpret_cast<int64_t *>(cb);
-            new_big[k] = cb ? reinterpret_cast<int64_t *>(cb + arc_bytes) : nullptr;
-            if (!cb) {
-                count_alloc_ok = false;
-                break;
-            }
+            new_big[k] = reinterpret_cast<int64_t *>(cb + r.arc_bytes);
             J.arc_cand_off = new_arc_off[k];
             J.big_list = new_big[k];
             J.result = d_results + k;
@@ -1723,25 +1731,13 @@ int Engine::step() {
         }
         if (chains.empty()) stage_bytes = align256(off_ctrinit + sizeof(int64_t) * dev::kCtrCount * n_couple_max);
     }
-    // layer runs: descriptors staged by (objectives, point type); per run what the host reads
-    // back (zeroed) and keep flags
+    // layer runs: descriptors staged by (objectives, point type)
     std::sort(runs.begin(), runs.end(), [](const RunSlot &a, const RunSlot &b) {
         return std::make_tuple(a.I->d, a.I->wide, a.meet, a.count_idx) <
                std::make_tuple(b.I->d, b.I->wide, b.meet, b.count_idx);
     });
     const size_t st_run = align256(stage_bytes);
     if (!runs.empty()) stage_bytes = st_run + sizeof(dev::RunJob) * runs.size();
-    const size_t run_out_bytes = align256(sizeof(dev::RunOut) * runs.size());
-    char *d_run = nullptr;
-    if (!runs.empty() && count_alloc_ok) {
-        size_t bytes = run_out_bytes;
-        for (RunSlot &r : runs) {
-            r.at_keep = bytes;
-            if (r.sd) bytes += align256(static_cast<size_t>(dev::kRunCap));
-        }
-        d_run = static_cast<char *>(scratch(bytes));
-        if (d_run == nullptr) count_alloc_ok = false;
-    }
     // Every device and pinned allocation of the step is made here, before any side moves
     // or launch, so that running out of memory rolls the step back and fails one request
     // instead of the engine.
@@ -1754,8 +1750,7 @@ int Engine::step() {
     // ... | the chain block | the terminal sizes of chained requests
     const size_t s_chain = align256(s_fin + sizeof(int32_t) * exps.size());
     const size_t s_chfin = s_chain + chain_dev_bytes;
-    const size_t s_run = align256(s_chfin + sizeof(int32_t) * chain_slots);
-    const size_t s_total = s_run + run_out_bytes;
+    const size_t s_total = s_chfin + sizeof(int32_t) * chain_slots;
     // oversized path: per group, the size-order list and the mark-path plan
     std::vector<int32_t *> big_order(glaunch.size(), nullptr);
     std::vector<void *> big_plan(glaunch.size(), nullptr);
@@ -1779,9 +1774,9 @@ int Engine::step() {
         }
     }
     if (!count_alloc_ok) {
-        // Out of device memory for bookkeeping: give everything back and fail the
-        // largest blocked request so the others can progress next step.
-        for (size_t k = 0; k < counts.size(); ++k) {
+        // Out of device memory for bookkeeping: give everything back, then plan again without
+        // layer runs, or fail the largest blocked request so the others can progress next step.
+        for (size_t k = 0; k < first_run_count; ++k) {  // (a run's counts are released with it)
             arena_.release(new_arc_off[k]);
             arena_.release(new_big[k]);
         }
@@ -1793,6 +1788,10 @@ int Engine::step() {
         for (RunSlot &r : runs) release_run(r);
         for (void *q : step_scratch_) arena_.release(q);
         step_scratch_.clear();
+        if (!runs.empty()) {
+            run_hold_ = kRunSkip;
+            return 0;
+        }
         // the request with the largest expansion of this step (else the last one counted)
         Instance *victim = counts.empty() ? nullptr : counts.back().I;
         int64_t most = -1;
@@ -1870,9 +1869,9 @@ int Engine::step() {
             J.sd_next = I.d_sd_next;
             J.sd_state = I.d_state;
             J.state_words = I.state_words;
-            J.keep = reinterpret_cast<uint8_t *>(d_run + r.at_keep);
+            J.keep = r.keep();
         }
-        J.out = reinterpret_cast<dev::RunOut *>(d_run) + k;
+        J.out = reinterpret_cast<dev::RunOut *>(d_fixed + f_run) + k;
         J.err = d_err_step;
         std::memcpy(hs + st_run + sizeof(dev::RunJob) * k, &J, sizeof(J));
     }
@@ -2108,7 +2107,6 @@ int Engine::step() {
         ktimes_.tile_launches += 1;
     }
     if (!runs.empty()) {
-        cudaMemsetAsync(d_run, 0, run_out_bytes, stream_);
         for (size_t i = 0; i < runs.size();) {
             size_t j = i + 1;
             while (j < runs.size() && runs[j].I->d == runs[i].I->d && runs[j].I->wide == runs[i].I->wide &&
@@ -2282,8 +2280,6 @@ int Engine::step() {
                                     sizeof(int32_t), cudaMemcpyDeviceToHost, stream_);
             }
     }
-    if (!runs.empty())
-        cudaMemcpyAsync(hsum + s_run, d_run, run_out_bytes, cudaMemcpyDeviceToHost, stream_);
     const double t_rel = trace_ ? now_s() : 0.0;
     for (void *q : to_release) arena_.release(q);
     const double t_enq = trace_ ? now_s() : 0.0;  // every copy and launch enqueued
@@ -2391,10 +2387,9 @@ int Engine::step() {
         RunSlot &r = runs[k];
         Instance &I = *r.I;
         I.in_run = false;
-        const dev::RunOut &o = reinterpret_cast<const dev::RunOut *>(hsum + s_run)[k];
+        const dev::RunOut &o = reinterpret_cast<const dev::RunOut *>(hsum + f_run)[k];
         if (I.phase != Instance::RUNNING) {  // cancelled or failed
             release_run(r);
-            for (size_t c = r.count_idx; c < r.count_idx + (r.meet ? 2 : 1); ++c) arena_.release(new_arc_off[c]);
             continue;
         }
         I.stats.kernel_expand_td_s += ms_expand * 1e-3;
@@ -2414,7 +2409,7 @@ int Engine::step() {
         I.stats.layers_td += o.done;
         I.stats.layers_bu += o.done_bu;
         I.stats.work_chained_layers += layers;
-        for (int side = 0; side < (r.meet ? 2 : 1); ++side) {
+        for (int side = 0; side < r.sides(); ++side) {
             Side &s = side == 0 ? I.td : I.bu;
             const int32_t done = side == 0 ? o.done : o.done_bu;
             const size_t c = r.count_idx + side;

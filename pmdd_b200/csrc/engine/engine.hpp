@@ -167,7 +167,8 @@ struct Instance {
 };
 
 // A request's layer run in one step (run.cu).  Two buffer sets per side, each one block: slot
-// offsets | sizes and sorted flags | points.
+// offsets | sizes and sorted flags | points | keep flags (state dominance).  Per side also the
+// count of the layer it stops before: per-arc offsets | oversized list.
 struct RunSlot {
     Instance *I = nullptr;
     bool meet = false;                  // method 3: both sides
@@ -178,14 +179,17 @@ struct RunSlot {
     bool sd = false;                    // with state dominance
     int32_t vcap = 0;                   // nodes of a layer the buffers hold
     int32_t max_nodes = 0, max_arcs = 0;  // of a layer the count may see
-    size_t pts_at = 0, at_keep = 0;
+    size_t pts_at = 0, keep_at = 0, arc_bytes = 0;
     char *buf[4] = {nullptr, nullptr, nullptr, nullptr};  // top-down sets, bottom-up sets
-    int sets() const { return meet ? 4 : 2; }
+    char *cnt[2] = {nullptr, nullptr};
+    int sides() const { return meet ? 2 : 1; }
+    int sets() const { return 2 * sides(); }
     int32_t *size(int b) const {
         return reinterpret_cast<int32_t *>(buf[b] + (sizeof(int64_t) * static_cast<size_t>(vcap) + 255) / 256 * 256);
     }
     uint8_t *sorted(int b) const { return reinterpret_cast<uint8_t *>(size(b) + vcap); }
     void *pts(int b) const { return buf[b] + pts_at; }
+    uint8_t *keep() const { return reinterpret_cast<uint8_t *>(buf[0] + keep_at); }
 };
 
 // Validates a flat DD and lays it out in an Instance (host side only).  The device copy
@@ -324,7 +328,8 @@ class Engine {
     void fail(Instance &I, int status, const std::string &msg);
     void release_instance(Instance &I);
     void release_side(Side &s);
-    // Picks the requests that run on from a small layer this step and gives them buffers.
+    // Picks the requests that run on from a small layer this step and gives them all the
+    // memory a run takes; without room, the request takes an ordinary step.
     void plan_runs(std::vector<RunSlot> &runs);
     void release_run(RunSlot &r);
     bool cuda_ok(cudaError_t e, const char *what);
@@ -378,6 +383,11 @@ class Engine {
     static constexpr int64_t kRunMaxRequests = 18;
     static constexpr int32_t kRunShared = 8;
     static constexpr int32_t kRunSkip = 4;
+    // A step's runs hold at most this share of the free memory, so that a tight budget is left
+    // to the ordinary steps' layers, and a step that runs out of memory with runs in it is
+    // planned again without (run_hold_ steps): runs cost no request its place.
+    static constexpr size_t kRunRoom = 64;
+    int32_t run_hold_ = 0;
     // Layer chaining (chain.cu): a request expanding by method 1 without state dominance
     // whose expansion in a step has at most chain_max_cand_ candidates goes on for more
     // layers in the same step, before the host reads back: chain_layers_ the first time,
