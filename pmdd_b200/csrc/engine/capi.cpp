@@ -737,7 +737,6 @@ pmdd_resident *pmdd_resident_build_knapsack(const pmdd_knapsack *ks, int32_t cou
             cudaStreamSynchronize(st) != cudaSuccess)
             return give_up(std::string("knapsack build failed: ") + cudaGetErrorString(cudaGetLastError()));
         E.count_launches(1);
-        std::vector<int64_t> runs_ints(1, 0);  // flatten scratch of each instance
         for (int32_t k = 0; k < m; ++k) {
             const pmdd_knapsack &q = ks[i0 + k];
             const int32_t Lc = q.n + 1;
@@ -769,30 +768,31 @@ pmdd_resident *pmdd_resident_build_knapsack(const pmdd_knapsack *ks, int32_t cou
             I->id = static_cast<uint64_t>(i0 + k);
             pmdd::layout_built_knapsack(I.get(), q.nobjs, bound > static_cast<int64_t>(INT32_MAX), layer_off, arc_at,
                                         q.n + 1);
+            if (I->A < I->N - 1) return give_up("knapsack build: inconsistent arc counts (internal)");
             I->dd = static_cast<unsigned char *>(E.alloc(I->dev_bytes));
             if (!I->dd) return give_up("built DD set does not fit the device memory budget");
-            runs_ints.push_back(runs_ints.back() + pmdd::dev::kp_run_ints(layer_off.back()));
+            E.bind_dd(*I, false);  // pointers only
             pmdd::dev::KpBuildJob &J = jobs[k];
+            J.first1 = I->d_out_off;
+            J.last1 = I->d_out_head;
+            J.first0 = I->d_out_w;
+            J.last0 = I->d_cursor;
             J.layer_offsets = reinterpret_cast<int32_t *>(I->dd + I->off_layer);
             J.in_arc_offsets = reinterpret_cast<int32_t *>(I->dd + I->off_in);
             J.arc_src = reinterpret_cast<int32_t *>(I->dd + I->off_src);
             J.arc_weight = reinterpret_cast<int32_t *>(I->dd + I->off_w);
             J.weights = reinterpret_cast<int32_t *>(I->dd + I->off_weights);
             J.min_weight = reinterpret_cast<int32_t *>(I->dd + I->off_minw);
+            J.degree = J.min_weight;
             J.sd_order = reinterpret_cast<int32_t *>(I->dd + I->off_sdord);
             R->bytes += static_cast<int64_t>(I->dev_bytes);
             R->tmpl.push_back(std::move(I));
             R->widths.push_back({ow, on, rw, rn});
         }
-        int32_t *d_runs = static_cast<int32_t *>(dev_alloc(sizeof(int32_t) * static_cast<size_t>(runs_ints[m])));
-        if (!d_runs) return give_up("knapsack build scratch does not fit the device memory budget");
-        for (int32_t k = 0; k < m; ++k) jobs[k].runs = d_runs + runs_ints[k];
         if (cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(jobs[0]) * m, cudaMemcpyHostToDevice, st) != cudaSuccess ||
             pmdd::dev::launch_kp_flatten(d_jobs, m, max_layers, st) != cudaSuccess)
             return give_up(std::string("knapsack flatten failed: ") + cudaGetErrorString(cudaGetLastError()));
         E.count_launches(2);
-        for (int32_t k = 0; k < m; ++k)
-            if (!E.bind_dd(*R->tmpl[i0 + k], false)) return give_up(E.ok() ? "out-arc CSR failed" : E.error());
         if (!E.build_csrs(R->tmpl, static_cast<size_t>(i0))) return give_up(E.ok() ? "out-arc CSR failed" : E.error());
         if (cudaMemcpyAsync(hhdr.data(), d_hdr, sizeof(int32_t) * hhdr.size(), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
@@ -803,9 +803,8 @@ pmdd_resident *pmdd_resident_build_knapsack(const pmdd_knapsack *ks, int32_t cou
         E.release(d_scr);
         E.release(d_hdr);
         E.release(d_jobs);
-        E.release(d_runs);
         temps.erase(std::remove_if(temps.begin(), temps.end(),
-                                   [&](void *p) { return p == d_scr || p == d_hdr || p == d_jobs || p == d_runs; }),
+                                   [&](void *p) { return p == d_scr || p == d_hdr || p == d_jobs; }),
                     temps.end());
         i0 = i1;
     }

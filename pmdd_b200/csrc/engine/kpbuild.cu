@@ -218,7 +218,8 @@ __global__ void __launch_bounds__(NT) kp_flatten_kernel(const KpBuildJob *jobs) 
     }
     const int32_t Kp = J.classes[l], Kc = J.classes[l + 1];
     const int32_t base = lo + Kp;
-    int32_t *s1 = J.runs + base, *e1 = s1 + N, *s0 = e1 + N, *e0 = s0 + N, *deg = e0 + N;
+    int32_t *s1 = J.first1 + base - 1, *e1 = J.last1 + base - 1, *s0 = J.first0 + base - 1, *e0 = J.last0 + base - 1;
+    int32_t *deg = J.degree + base - 1;
     int32_t *longs = J.idx + l * S;  // children with a long run (the states are done with)
     const int32_t *cnew = J.cls_new + l * S, *c0 = J.cls_c0 + l * S, *c1 = J.cls_c1 + l * S;
     for (int32_t v = tid; v < Kc; v += NT) {

@@ -48,7 +48,10 @@ struct KpBuildJob {
     int32_t *classes;        // [n+1] reduced layer sizes
     int32_t *arcs_into;      // [n+1] arcs into each layer
     int32_t *err;            // 0 ok; 1 inconsistent counts; 2 min_weight order check failed
-    int32_t *runs;           // kp_flatten_kernel scratch: kp_run_ints(nodes)
+    // kp_flatten_kernel scratch, N - 1 ints each (the nodes below the root): the first and last
+    // parent class of either arc type, and the in-degree.  Arrays of the flat DD and its
+    // out-arc CSR that are written later serve (arcs >= N - 1, every node but the root has one)
+    int32_t *first1, *last1, *first0, *last0, *degree;
     // the flat DD (kp_flatten_kernel), pmdd_dd layout
     int32_t *layer_offsets, *in_arc_offsets, *arc_src, *arc_weight, *weights, *min_weight, *sd_order;
 };
@@ -58,10 +61,6 @@ inline int64_t kp_scratch_ints(int32_t n, int32_t cap) {
     const int64_t S = static_cast<int64_t>(cap) + 1;
     return (4 * (static_cast<int64_t>(n) + 1) + 10) * S;
 }
-
-// Flatten scratch of a DD of N nodes: per node the first and last parent class of either arc
-// type, and its in-degree.
-inline int64_t kp_run_ints(int32_t N) { return 5 * static_cast<int64_t>(N); }
 
 cudaError_t launch_kp_reduce(const KpBuildJob *jobs, int count, cudaStream_t stream);
 cudaError_t launch_kp_flatten(const KpBuildJob *jobs, int count, int max_layers, cudaStream_t stream);

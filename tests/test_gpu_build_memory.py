@@ -1,0 +1,45 @@
+"""Device memory of building sets: a knapsack set is built in a budget that holds the diagrams
+and the construction's state arrays."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT
+
+pytestmark = pytest.mark.gpu
+
+BUILD = r"""
+import sys
+sys.path.insert(0, {root!r})
+import numpy as np
+import pmdd_b200 as P
+from pmdd_b200 import instances
+ks = [instances.knapsack_arrays(60, 2, 90 + i) for i in range({count})]
+s = P.ResidentSet.from_knapsack(ks)
+print(s.device_bytes, sum(s.dd_info(i)["num_nodes"] for i in range({count})))
+"""
+
+def _child(code, count, arena):
+    env = dict(os.environ)
+    env.pop("PMDD_ARENA_BYTES", None)
+    if arena:
+        env["PMDD_ARENA_BYTES"] = str(arena)
+    return subprocess.run([sys.executable, "-c", code.format(root=ROOT, count=count)], env=env, capture_output=True,
+                          text=True, timeout=300)
+
+
+def test_knapsack_build_takes_no_more_than_the_diagrams_and_state_arrays():
+    from pmdd_b200 import instances
+
+    count = 6
+    ks = [instances.knapsack_arrays(60, 2, 90 + i) for i in range(count)]
+    state = sum(4 * (4 * 61 + 10) * (int(cap) + 1) for _, _, cap in ks)
+    p = _child(BUILD, count, 0)
+    assert p.returncode == 0, p.stderr
+    nbytes, nodes = map(int, p.stdout.split())
+    small = 64 * 1024 * count  # inputs, headers, descriptors, rounding
+    assert small < 20 * nodes / 4 and nbytes + state > 80 << 20
+    p = _child(BUILD, count, nbytes + state + small)
+    assert p.returncode == 0, p.stderr
