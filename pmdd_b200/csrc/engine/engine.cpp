@@ -880,7 +880,13 @@ bool Engine::build_csrs(const std::vector<std::unique_ptr<Instance>> &insts, siz
     }
     if (jobs.empty()) return true;
     void *d = arena_.alloc(sizeof(dev::CsrJob) * jobs.size());
-    if (!d) return false;
+    if (!d) {  // no room for the list: one DD at a time
+        for (const dev::CsrJob &j : jobs) {
+            if (!cuda_ok(dev::launch_build_out_csr(j, stream_), "out-arc CSR")) return false;
+            count_launches(dev::kCsrLaunches);
+        }
+        return true;
+    }
     // (the copy from pageable memory has left `jobs` when it returns)
     const bool ok = cuda_ok(cudaMemcpyAsync(d, jobs.data(), sizeof(dev::CsrJob) * jobs.size(), cudaMemcpyHostToDevice,
                                             stream_),

@@ -1,5 +1,5 @@
-"""Device memory of building sets: a knapsack set is built in a budget that holds the diagrams
-and the construction's state arrays."""
+"""Device memory of building and uploading sets: a knapsack set is built, and a set of diagrams
+uploaded, in a budget that holds the diagrams and the construction's state arrays."""
 import os
 import subprocess
 import sys
@@ -20,6 +20,17 @@ ks = [instances.knapsack_arrays(60, 2, 90 + i) for i in range({count})]
 s = P.ResidentSet.from_knapsack(ks)
 print(s.device_bytes, sum(s.dd_info(i)["num_nodes"] for i in range({count})))
 """
+
+UPLOAD = r"""
+import sys
+sys.path.insert(0, {root!r})
+import pmdd_b200 as P
+from pmdd_b200 import instances
+dd = P.DecisionDiagram.from_text(instances.knapsack_text(24, 2, 90), 1, 2)
+s = P.ResidentSet([dd] * {count})
+print(s.device_bytes)
+"""
+
 
 def _child(code, count, arena):
     env = dict(os.environ)
@@ -42,4 +53,13 @@ def test_knapsack_build_takes_no_more_than_the_diagrams_and_state_arrays():
     small = 64 * 1024 * count  # inputs, headers, descriptors, rounding
     assert small < 20 * nodes / 4 and nbytes + state > 80 << 20
     p = _child(BUILD, count, nbytes + state + small)
+    assert p.returncode == 0, p.stderr
+
+
+def test_upload_takes_no_more_than_the_diagrams():
+    p = _child(UPLOAD, 1, 0)
+    assert p.returncode == 0, p.stderr
+    one = (int(p.stdout) + 255) // 256 * 256
+    count = (80 << 20) // one + 1
+    p = _child(UPLOAD, count, one * count)
     assert p.returncode == 0, p.stderr
