@@ -142,7 +142,8 @@ typedef struct pmdd_stats {
     int64_t work_stair_candidates_total; /* three objectives: candidates of tile destinations above the
                                             pairwise limit, filtered by staircases */
     int64_t work_chained_layers;         /* layers expanded by chained steps (several layers between two
-                                            host read-backs, for steps with few candidates) */
+                                            host read-backs, for steps with few candidates);
+                                            layer runs count in pmdd_run_layer_count only */
 } pmdd_stats;
 
 /* ------------------------------------------------------------ one-shot entry
@@ -331,6 +332,9 @@ void pmdd_server_destroy(pmdd_server *srv);
 const char *pmdd_version(void);
 /* Number of kernels this library has launched in this process (all calls). */
 int64_t pmdd_launch_count(void);
+/* Number of layers this library has expanded in layer runs (the small layers of a request
+ * that follow one another inside one launch) in this process. */
+int64_t pmdd_run_layer_count(void);
 /* The oversized-destination crossover (candidates from which a destination is filtered
  * by the GPU-wide pass rather than one sort-filter-skyline block) that the tuning file
  * at `path` holds for (nobjs, problem_type), or 0 if it holds none (engines then use their

@@ -229,6 +229,7 @@ GPU_SYMBOLS = {
     "pmdd_server_inject_alloc_failures": (ctypes.c_int, [ctypes.c_void_p, c_i64, c_i64]),
     "pmdd_version": (ctypes.c_char_p, []),
     "pmdd_launch_count": (c_i64, []),
+    "pmdd_run_layer_count": (c_i64, []),
     "pmdd_tuned_mark_min": (c_i64, [ctypes.c_char_p, c_i32, c_i32]),
     "pmdd_tuned_lex_pair_max": (c_i64, [ctypes.c_char_p, c_i32, c_i32]),
     "pmdd_tuned_tile_window_max": (c_i64, [ctypes.c_char_p, c_i32, c_i32]),

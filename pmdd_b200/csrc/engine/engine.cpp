@@ -1071,6 +1071,7 @@ struct ChainGroup {
 }  // namespace
 
 std::atomic<int64_t> g_total_launches{0};
+std::atomic<int64_t> g_total_run_layers{0};
 
 void Engine::release_run(RunSlot &r) {
     for (char *b : r.buf) arena_.release(b);
@@ -2414,7 +2415,6 @@ int Engine::step() {
         I.stats.dominance_filtered_total += o.removed;
         I.stats.layers_td += o.done;
         I.stats.layers_bu += o.done_bu;
-        I.stats.work_chained_layers += layers;
         for (int side = 0; side < r.sides(); ++side) {
             Side &s = side == 0 ? I.td : I.bu;
             const int32_t done = side == 0 ? o.done : o.done_bu;
@@ -2461,7 +2461,7 @@ int Engine::step() {
             I.stats.work_frontier_peak_points = std::max(I.stats.work_frontier_peak_points, I.td.res.cur_total);
         }
     }
-    chained_layers_total_ += run_layers;
+    g_total_run_layers += run_layers;
     for (size_t k = 0; k < ujobs.size(); ++k) {
         Instance &I = *ujob_inst[k];
         if (I.phase == Instance::DONE) continue;
@@ -2578,7 +2578,6 @@ int Engine::step() {
             }
         }
     }
-    chained_layers_total_ += chained_done;
     if (!fetches.empty()) {
         size_t total = 0;
         for (auto &f : fetches) total += align256(f.first->result.size());

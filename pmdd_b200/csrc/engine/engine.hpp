@@ -30,6 +30,8 @@ double now_s();
 
 // Kernels launched by every engine of this process.
 extern std::atomic<int64_t> g_total_launches;
+// Layers they expanded in layer runs.
+extern std::atomic<int64_t> g_total_run_layers;
 
 // First-fit allocator over device memory taken in a few large cudaMalloc chunks, the
 // first of `initial` bytes at start-up and more (doubling, at most 16 GB at a time) when
@@ -402,7 +404,6 @@ class Engine {
     bool chain_grow_all_ = false;
     int64_t chain_max_requests_ = 128;
     int64_t chain_max_cand_ = int64_t(1) << 17;
-    int64_t chained_layers_total_ = 0;  // layers expanded by chained steps (statistics)
     int32_t lex_pair_max_fixed_ = -1;
     std::map<std::pair<int, int>, int64_t> tuned_pair_max_;
     int32_t pair_max_for(int d, int problem_type) const;
