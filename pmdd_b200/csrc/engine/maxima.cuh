@@ -71,7 +71,7 @@ struct SegHead {
     uint32_t scale[D];                // bin = (x - mn >> shift) * scale >> 16
     int32_t shift[D];
     uint32_t piv_idx[kMaxPivots];
-    uint8_t lut[D][kMaxBins];         // bin -> rank, 8 bits
+    alignas(4) uint8_t lut[D][kMaxBins];  // bin -> rank, 8 bits
     SortedPt<D, T> piv[kMaxPivots];
 };
 
@@ -393,7 +393,7 @@ template <int D, typename T, class Src>
 __global__ void __launch_bounds__(kMaxThreads) maxima_prefilter_kernel(Src src) {
     __shared__ SortedPt<D, T> s_piv[kMaxPivots];
     __shared__ uint32_t s_idx[kMaxPivots];
-    __shared__ uint8_t s_lut[D][kMaxBins];
+    __shared__ alignas(4) uint8_t s_lut[D][kMaxBins];  // copied a word at a time
     int h;
     int64_t base;
     if (!src.chunk(blockIdx.x, &h, &base)) return;
