@@ -49,12 +49,9 @@ __host__ __device__ constexpr bool tile_resident(int64_t candidates, int64_t arc
 }
 
 constexpr int kCountThreads = 1024;
-constexpr int kBigThreads = 256;
-constexpr int kBigJTile = 1024;       // candidates per shared-memory comparison tile
 
-// Device error word bits (written with atomicOr; read back once per step).
+// Device error word (written with atomicOr; read back once per step).
 constexpr uint32_t kErrBounds = 1u;        // an index check failed (work skipped)
-constexpr uint32_t kErrCoupleOverflow = 2u;
 
 // One layer expansion of one instance in one direction.  "Items" are the destination
 // nodes of the layer; each has a contiguous range of arcs whose neighbour (the arc's

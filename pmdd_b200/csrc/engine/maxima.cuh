@@ -63,9 +63,7 @@ constexpr int kMaxBins = 256;
 template <int D, typename T>
 struct SegHead {
     uint32_t rows;                    // points the pivots left
-    int32_t bits;                     // key bits; 2^bits buckets
     int32_t npiv;
-    int32_t pad;
     T mn[D];
     uint32_t range[D];                // sampled range, shifted right by shift
     uint32_t scale[D];                // bin = (x - mn >> shift) * scale >> 16
@@ -385,7 +383,6 @@ __global__ void __launch_bounds__(kMaxStatThreads) maxima_stats_kernel(Src src) 
         int kept = 0;
         for (int j = 0; j < np; ++j) kept += s_drop[j] ? 0 : 1;
         v.head->npiv = kept;
-        v.head->bits = v.bits;
     }
 }
 

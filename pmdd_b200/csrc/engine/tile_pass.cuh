@@ -154,7 +154,7 @@ __device__ __forceinline__ int stage_items(TileItems &S, const ExpandJob &J, Run
             if (J.out_sorted) J.out_sorted[i] = (c == 0 || (resident && in_order)) ? 1 : 0;
             S.item_c0[k] = s;
             S.item_a0g[k] = a0;
-                if (resident) {
+            if (resident) {
                 cnt[r] = static_cast<int32_t>(c);
                 narc[r] = a1 - a0;
             }
