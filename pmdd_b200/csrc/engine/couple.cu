@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) out_scatter_kernel(const CsrJob *__restri
 static cudaError_t launch_csr(const CsrJob *jobs, const CsrJob &one, int count, int32_t max_nodes, int32_t max_arcs,
                               cudaStream_t stream) {
     if (count <= 0) return cudaSuccess;
-    const int cap = std::max(1, 1184 / std::min(count, 64));
+    const int cap = std::max(1, 148 * 8 / std::min(count, 64));  // 8 blocks per SM over the set
     const dim3 gn(std::min(cap, max_nodes / 256 + 1), count), ga(std::min(cap, max_arcs / 256 + 1), count);
     csr_zero_kernel<<<gn, 256, 0, stream>>>(jobs, one);
     out_degree_kernel<<<ga, 256, 0, stream>>>(jobs, one);

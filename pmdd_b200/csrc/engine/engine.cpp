@@ -1081,7 +1081,7 @@ void Engine::release_run(RunSlot &r) {
 
 void Engine::plan_runs(std::vector<RunSlot> &runs) {
     for (auto &p : active_) p->in_run = false;
-    if (run_layers_ <= 0 || chain_layers_ <= 0 || static_cast<int64_t>(active_.size()) > kRunMaxRequests) return;
+    if (run_layers_ <= 0 || chain_layers_ <= 0 || static_cast<int64_t>(active_.size()) > run_max_requests()) return;
     if (run_hold_ > 0) {
         --run_hold_;
         return;

@@ -376,13 +376,17 @@ class Engine {
     // has at most kRunEnter candidates, goes on layer by layer in one launch (method 3: by
     // the side rule, without state dominance): up to run_layers_ layers
     // (PMDD_RUN_LAYERS, 0: off) when nothing else is under way, else kRunShared, since the
-    // others wait for the step.  A run that stops at once is not tried again for kRunSkip
-    // steps.  With more than kRunMaxRequests requests (one cluster of 8 per 8 SMs) the
-    // ordinary steps, whose launches they share, are faster: the 192-instance stream takes 94
-    // ms without runs and 102 ms with, a served burst of 48 requests 48 and 54 ms.
+    // others wait for the step.  Sets of 1, 4 and 12 small requests by method 1 are up to 1.2
+    // times as slow with kRunEnter 2048 and up to 1.3 times with 16384; a run that stops at
+    // once is not tried again for kRunSkip steps (1, 4 and 16 are level).  Runs are for steps
+    // of at most run_max_requests() requests, whose clusters all fit the chip at once: sets of
+    // 1 to 18 knapsack, set-packing or TSP requests are 1.02 to 4.2 times as fast with runs as
+    // without.  With more of them the ordinary steps, whose launches they share, are faster:
+    // the 192-instance stream takes 94 ms without runs and 102 ms with, a served burst of 48
+    // requests 48 and 54 ms.
     int32_t run_layers_ = 1 << 20;
     static constexpr int64_t kRunEnter = 8192;
-    static constexpr int64_t kRunMaxRequests = 18;
+    int64_t run_max_requests() const { return sms_ / dev::kRunBlocks; }  // 18
     static constexpr int32_t kRunShared = 8;
     static constexpr int32_t kRunSkip = 4;
     // A step's runs hold at most this share of the free memory, so that a tight budget is left
