@@ -37,7 +37,7 @@ enum pmdd_status {
     PMDD_ERR_CUDA = 2,           /* CUDA runtime error (text in err) */
     PMDD_ERR_OOM = 3,            /* request cannot fit the device / server budget */
     PMDD_ERR_CAND_OVERFLOW = 4,  /* a single destination exceeds what one pass can hold */
-    PMDD_ERR_TIMEOUT = 5,        /* a bounded device wait gave up */
+    PMDD_ERR_TIMEOUT = 5,        /* a bounded device wait gave up (no call returns it at present) */
     PMDD_ERR_INTERNAL = 6,       /* device-side consistency check failed */
     PMDD_ERR_CANCELLED = 7,      /* request cancelled before completion */
     PMDD_ERR_NO_DEVICE = 8,      /* no CUDA device / extension not usable */
@@ -338,7 +338,8 @@ int64_t pmdd_run_layer_count(void);
 /* The oversized-destination crossover (candidates from which a destination is filtered
  * by the GPU-wide pass rather than one sort-filter-skyline block) that the tuning file
  * at `path` holds for (nobjs, problem_type), or 0 if it holds none (engines then use their
- * built-in crossover, 1025: every destination too large for a tile).  path NULL: the file
+ * built-in crossover, 1025: every destination too large for a tile; they take a smaller
+ * value as 1025).  path NULL: the file
  * engines read at start-up (PMDD_TUNING_FILE, else the per-user cache written by
  * pmdd_b200.autotune).  No counterpart in the reference, which has one filter path. */
 int64_t pmdd_tuned_mark_min(const char *path, int32_t nobjs, int32_t problem_type);

@@ -21,10 +21,10 @@
 // The pass replaced one that tested every candidate against 4*sqrt(n) pivots and then
 // compared all pairs of the rest (one B200, oversized path per enumeration, before -> now):
 // TSP d=5 n=13 38.7 -> 9.6 ms (23.7 M candidates), KP d=4 n=60 18.8 -> 6.0 ms (17.7 M),
-// KP d=7 n=25 1.14 -> 0.56 ms.  It also took over the three-objective destinations with
-// sorted runs, which one staircase warp each walked in lexicographic order: oversized
-// path of the 192-instance stream 21.3 -> 11.9 ms, against 2 ms more in the tiles, whose
-// runs from these parents arrive unsorted.
+// KP d=7 n=25 1.14 -> 0.56 ms, the 192-instance stream 31.4 -> 11.2 ms, where it also took
+// over the three-objective destinations with sorted runs, which one staircase warp each
+// walked in lexicographic order (against 2 ms more in the tiles, whose runs from these
+// parents arrive unsorted).
 #include "big_common.cuh"
 #include "kernels.cuh"
 #include "maxima.cuh"

@@ -31,10 +31,11 @@
 // second.  It replaced one staircase warp per 64-candidate segment, whose walks were serial
 // chains of shuffles (51 % of the kernel's time, its warps 61 % busy): 1.68 G -> 0.93 G warp
 // instructions on a captured launch of the 192-instance stream.  The kernel waits on
-// barriers, shared-memory latency and dependent loads, not on a unit (issue slots 56 % busy,
-// ALU 51 %): tile time of that stream's 684 M candidates 73.8 ms before, 49.7 ms with the
+// barriers, shared-memory latency and dependent loads, not on a unit (issue slots 53 % busy,
+// ALU 50 %): tile time of that stream's 684 M candidates 73.8 ms before, 49.7 ms with the
 // chunk filter at 512 threads and 79 KB, 40.3 ms with four blocks of 256 threads per SM,
-// the merge in place and the next tile fetched ahead (one B200).
+// the merge in place and the next tile fetched ahead, 38.3 ms with the sorts of kMergeRuns
+// (one B200).
 //
 // The keep rule is the reference GPU filter's (src/pmdd/enum/gpu/dominance_utils.cuh:
 // 10-23): q is dropped iff another candidate p of the destination has p >= q on every
@@ -48,8 +49,9 @@
 namespace pmdd {
 namespace dev {
 
-// 256 threads and 55 KB of shared memory (int32): four blocks share an SM, so that one
-// block's barriers and dependent loads are covered by the others.
+// 256 threads and 54 KB of shared memory (int32): four blocks share an SM, so that one
+// block's barriers and dependent loads are covered by the others (64 registers, 20 bytes of
+// them spilled).  int64 points take 95 KB: two blocks of 128 registers.
 constexpr int kLexThreads = 256;
 // Destinations of more than kMergeRuns runs are sorted in shared memory instead of merged
 // (a search per other run: hundreds on the last layers of a knapsack), and so are runs of

@@ -39,8 +39,10 @@
 namespace pmdd {
 namespace dev {
 
-// Points of 16 bytes leave 57 KB per block: four blocks of 256 threads share an SM; larger
-// points 89 KB and more, two blocks of 512.
+// Points of 16 bytes make 61 KB a block: three blocks of 256 threads share an SM; points of 32
+// bytes 93 KB, two blocks of 512; larger ones (int64, five objectives and more) 125-157 KB, one.
+// The launch bounds ask for four or two, which holds every instance at 64 registers (int64
+// points of five objectives and more spill 4-22 bytes, int32 ones of eight 8).
 template <int D, typename T>
 constexpr int pair_threads() {
     return sizeof(PackedPt<D, T>) <= 16 ? 256 : 512;

@@ -2,9 +2,8 @@
 // one copy of each (ParetoFrontier::merge semantics, src/pmdd/enum/pareto_frontier.hpp:
 // 237-303).  Sets of at most kParetoBlockMax points take the block-wide sort-filter-skyline
 // sweep of sfs.cuh (one launch), larger ones the GPU-wide pass of maxima.cuh as its one
-// segment: a host call on 32768 points of 4 objectives
-// takes 0.2 ms instead of 11 ms with the one block, on 131072 of 5 objectives 0.7 ms instead
-// of 1.05 s.
+// segment: a host call on 32768 points of 4 objectives takes 0.15 ms instead of 11 ms with the
+// one block, on 131072 of 5 objectives 0.7 ms instead of 1.05 s.
 #include "kernels.cuh"
 #include "maxima.cuh"
 #include "pareto.cuh"
@@ -19,7 +18,10 @@ namespace {
 
 // Below, one block's single launch wins over the six of the GPU-wide pass, whose fixed cost is
 // about 20 us: a call on 300 points takes 78-93 us by the block, on 600 points 165-203 us,
-// on 1025 points by the GPU-wide pass 84-112 us (d = 2 .. 7, host call included).
+// on 1025 points by the GPU-wide pass 84-112 us (d = 2 .. 7, host call included).  The block's
+// time goes with the maxima, which nothing tells beforehand: where a handful of points lies
+// above nearly all others it stays ahead up to some 8000 points (50-120 us against 70-140 us),
+// where most points are maxima it takes 0.4 ms for 1025 and 4-6 ms for 4097.
 constexpr int64_t kParetoBlockMax = 320;
 
 struct OneSrc {

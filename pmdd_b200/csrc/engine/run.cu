@@ -20,12 +20,12 @@
 // alternate, so a line of the layer before last may still be there.
 //
 // One B200, a layer: about 10 us, a chain of dependent loads, block barriers and the
-// cluster's, against 23 us for the two launches of a chained one.  KP d=3 n=20: 21 layers
-// in 0.21 ms (call 0.77 -> 0.32 ms); set packing d=3 n=100: 1.1 ms (3.0 -> 1.27 ms); n=91
-// with state dominance, which ordinary steps take one layer at a time: 2.2 ms (8.9 -> 3.1
-// ms, of which 1.5 ms since the orders are counting-sorted at preparation; 2.7 ms before a
-// node's loads went out together, its partners' labels 32 at a time, and nodes that lose
-// no label were left out of the compaction).
+// cluster's, against 23 us for the two launches of a chained one.  KP d=3 n=20: 20 layers
+// in 0.22 ms (call 0.74 -> 0.33 ms); a set packing d=3 n=100 whose layers all fit: 1.1 ms
+// (call 3.0 -> 1.3 ms; 1.6 - 1.9 ms where layers in its middle outgrow the regions); n=91 with
+// state dominance, which ordinary steps take one layer at a time: 2.2 ms (call 9.0 -> 2.7 -
+// 3.2 ms; a node's loads out together, its partners' labels 32 at a time, and no compaction
+// of nodes that lose no label are 0.5 ms of it).
 #include "run.cuh"
 
 #include <cooperative_groups.h>
