@@ -9,9 +9,8 @@ import sys
 import numpy as np
 import pytest
 
-import oracle
 import pmdd_b200 as P
-from conftest import ROOT, frontier_digest
+from conftest import ROOT
 from pmdd_b200 import instances
 
 pytestmark = pytest.mark.gpu
